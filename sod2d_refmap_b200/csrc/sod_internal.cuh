@@ -81,7 +81,7 @@ struct DevParams {
   double g_gm1, inv_gm1, inv_Rgas;  // gamma/(gamma-1), 1/(gamma-1), 1/Rgas (host-computed)
   double CpPr, Cp09;                 // Cp/Prt, Cp/0.9 (host-computed)
   // FP32 copies for the mixed kernels (host-converted: FP64->FP32 conversions are slow on the GPU)
-  float gamma_f, c_rho_f, c_ener_f, CpPr_f, Cp09_f;  // gamma, c_rho, c_ener, Cp/Prt, Cp/0.9
+  float gamma_f, c_rho_f, c_ener_f, CpPr_f, Cp09_f, inv_gm1_f;  // gamma, c_rho, c_ener, Cp/Prt, Cp/0.9, 1/(gamma-1)
   int flag_les;
   double c_sgs;
   int total_enthalpy;  // flag_total_enthalpy: energy convection of full_convec_ijk_H

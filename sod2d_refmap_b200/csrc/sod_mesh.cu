@@ -341,6 +341,7 @@ static void to_dev_params(const SodParams* s, DevParams* d) {
   d->c_ener_f = (float)s->c_ener;
   d->CpPr_f = (float)(s->Cp / s->Prt);
   d->Cp09_f = (float)(s->Cp / 0.9);
+  d->inv_gm1_f = (float)(1.0 / (s->gamma_gas - 1.0));
 }
 
 int sod_mesh_set_params(SodMesh* m, const SodParams* p) {
