@@ -7,18 +7,19 @@
 // viscosity mu_e is frozen at its forward value (it is updated once per step from the state
 // after the step, time_integ.f90:492-493), as is dt.
 //
-// k_rhs_vjp (one element per CTA, one thread per gauss point, FP64) recomputes the forward
-// derivative quantities, then runs the reverse sweep:
-//   diffusion  output seeds -> D applied along lines (the transpose of pass 2's D^T) ->
-//              contravariant-flux adjoints -> stress/heat-flux adjoints
-//   convection the split-form combination reversed pointwise
-//   both       derivative adjoints mapped back with He^T and D^T along lines to nodal product
-//              fields, then the product rule, the EOS and u = q/rho in reverse.
-// The energy convection is linear in (h, k) through h + k only (every h term has a k twin with
-// the same structure), so the adjoint works with the total enthalpy H = h + k; q (x) u is
-// symmetric (rho u_c u_j), so its 9 components reduce to 6 like u (x) u.  The 29 nodal adjoint
-// fields go through shared memory in chunks of kChunk fields (3 line arrays each), which keeps
-// the CTA at 21 KB of shared memory.
+// k_rhs_vjp: one element per CTA, one thread per gauss point, FP64.  The convection of the stage
+// residual is a sum over line pairs (the two-point form of the quartets, see sod_rhs.cu):
+//   R_mass(x) = 1/2 sum_dir sum_l D[x][l] (rho_x + rho_l) (V_x + V_l),   V_l = sum_c He(c,dir)(x) u_c(l)
+//   R_f(x)    = 1/4 sum_dir sum_l D[x][l] (rho_x + rho_l) (V_x + V_l) (f_x + f_l),  f = u_c, H = h + k
+// so a node's adjoint is one pass over its 12 line points, each taken in both roles: the node as
+// the output point x (row D[a][l], own metric and seeds) and as the partner l (column D[l][a], the
+// line point's metric and seeds).  That needs the line point's 6 fields, 5 seeds and 3 metric
+// values and ~42 FP64 operations; q, rho H and the product fields carry no adjoint of their own.
+// The same pass structure gives the forward gradients and the D-line sums of the seeds (the
+// transpose of pass 2's D^T); the viscous stress is reversed pointwise and its five gradient
+// fields (u, rho, T) go back through He^T and D^T.  32^3, one launch: 219 us; 467 us with the 29 nodal
+// product fields each sent back through three line arrays.  Bounded by FP64 latency at 12 resident
+// warps per SM (168 registers; FP64 pipe ~55% busy).
 // Element-node adjoints are assembled by the same ordered CSR gather as the forward path.
 #include "sod_internal.cuh"
 #include <cmath>
@@ -33,18 +34,11 @@ namespace adj {
 
 constexpr double kC1 = 0.000001458;
 constexpr double kS = 110.4;
-// forward fields staged in shared memory (H = h + k total enthalpy); the products rho H, H u and
-// u (x) u are formed from them at the line points
-enum { F_RHO = 0, F_H, F_T, F_U0, F_U1, F_U2, F_Q0, F_Q1, F_Q2, NF_FWD };
-// nodal adjoint fields receiving D^T line sums: 11 gradient fields, rho H u and H u (divergence),
-// q (x) u and u (x) u (symmetric, divergence by rows)
-enum { A_RHO = 0, A_P, A_H, A_RH, A_T, A_U0, A_U1, A_U2, A_Q0, A_Q1, A_Q2,
-       A_FE0, A_FE1, A_FE2, A_FUE0, A_FUE1, A_FUE2,
-       A_F00, A_F01, A_F02, A_F11, A_F12, A_F22,
-       A_UU00, A_UU01, A_UU02, A_UU11, A_UU12, A_UU22, NF_ADJ };
-constexpr int kChunk = 10;
-constexpr int kArrays = 3 * kChunk;  // >= NF_FWD + 6 (forward phase) and >= 6 (seed phase)
-static_assert(kArrays >= NF_FWD + 6, "shared arrays");
+// shared arrays: nodal fields; seeds over Ml (2 w_mass, w_energy, w_mom x3), nu_e w_mass, kappa
+// w_energy; gpvol He (3c + dir); then the contravariant grad rho and grad T.  The adjoint line
+// arrays of the five gradient fields (x3 directions) overlay the first 15 once they are read.
+enum { F_RHO = 0, F_H, F_T, F_U0, F_U1, F_U2, W_M2, W_E, W_O0, W_O1, W_O2, W_NU, W_KE, F_G, F_V6 = F_G + 9, NF_ALL = F_V6 + 6 };
+constexpr int kDtab = 32;  // D rows, then D^T rows
 
 struct VjpArgs {
   int nelem;
@@ -65,357 +59,305 @@ struct VjpArgs {
   DevParams prm;
 };
 
-__device__ __forceinline__ void giso_line(const double* f, int i, int j, int k, const double (&D)[NP1][NP1],
-                                          double& gx, double& gy, double& gz) {
-  gx = D[i][0] * f[sidx(0, j, k)] + D[i][1] * f[sidx(1, j, k)] + D[i][2] * f[sidx(2, j, k)] + D[i][3] * f[sidx(3, j, k)];
-  gy = D[j][0] * f[sidx(i, 0, k)] + D[j][1] * f[sidx(i, 1, k)] + D[j][2] * f[sidx(i, 2, k)] + D[j][3] * f[sidx(i, 3, k)];
-  gz = D[k][0] * f[sidx(i, j, 0)] + D[k][1] * f[sidx(i, j, 1)] + D[k][2] * f[sidx(i, j, 2)] + D[k][3] * f[sidx(i, j, 3)];
+__device__ __forceinline__ void load4(const double* p, double (&w)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
 }
 
-// sum_m D[m][i] fx(m,j,k) + D[m][j] fy(i,m,k) + D[m][k] fz(i,j,m)
-__device__ __forceinline__ double divT_line(const double* fx, const double* fy, const double* fz, int i, int j, int k,
-                                            const double (&D)[NP1][NP1]) {
-  double s = 0.0;
-#pragma unroll
-  for (int m = 0; m < NP1; ++m)
-    s += D[m][i] * fx[sidx(m, j, k)] + D[m][j] * fy[sidx(i, m, k)] + D[m][k] * fz[sidx(i, j, m)];
-  return s;
-}
+// Keeps the line passes apart: without it the compiler carries the line values of one pass over to
+// the next in registers (up to 192 doubles) and spills them.
+__device__ __forceinline__ void pass_fence() { asm volatile("" ::: "memory"); }
 
-// symmetric pair (c, j) of each q(x)u / u(x)u field, in enum order 00 01 02 11 12 22
-__device__ constexpr int sym_c(int t) { return t < 3 ? 0 : (t < 5 ? 1 : 2); }
-__device__ constexpr int sym_j(int t) { return t < 3 ? t : (t < 5 ? t - 2 : 2); }
-
+// Resident CTAs per SM the register budget must allow: 6 (168 registers, no spill) 0.282 ms for the whole
+// call at 32^3, 8 (128 registers, 92 bytes of spill) 0.297 ms.
 #ifndef SOD_VJP_MIN_BLOCKS
-#define SOD_VJP_MIN_BLOCKS 1  // CTAs per SM the register allocation must allow
+#define SOD_VJP_MIN_BLOCKS 6
 #endif
 // TOTH: flag_total_enthalpy (energy convection of full_convec_ijk_H)
 template <bool TOTH>
 __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArgs a) {
-  __shared__ __align__(16) double sm[kArrays * FSTRIDE];
-  __shared__ DMat Ds;
-  const int e = blockIdx.x, d = threadIdx.x;
-  const int i = d & 3, j = (d >> 2) & 3, k = d >> 4, s = sidx(i, j, k);
-  if (d < 16) Ds.d[d >> 2][d & 3] = a.D.d[d >> 2][d & 3];
+  __shared__ __align__(16) double sm[NF_ALL * FSTRIDE];
+  __shared__ __align__(16) double dtab[kDtab];
+  const int e = blockIdx.x, lt = threadIdx.x;
+  // lane bits (i0 j0 i1 j1 k): one shared-memory wavefront per xi and eta line load (see sod_rhs.cu)
+  const int i = (lt & 1) | ((lt >> 1) & 2), j = ((lt >> 1) & 1) | ((lt >> 2) & 2), k = lt >> 4;
+  const int d = i + 4 * j + 16 * k, s = sidx(i, j, k);
+  if (lt < 32) dtab[lt] = lt < 16 ? a.D.d[lt >> 2][lt & 3] : a.D.d[lt & 3][(lt >> 2) & 3];
   const double* Ge = a.geo + (size_t)e * NGEO * NN;
-  double H[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) H[c] = Ge[c * NN + d];
-  const double gpv = Ge[9 * NN + d];
   const int n = a.econn[(size_t)e * NN + d];
-  const double g = a.prm.gamma, Rg = a.prm.Rgas;
+  const int64_t N = a.npoin;
+  const double g = a.prm.gamma;
   const double rho = a.rho[n];
   const double qv[3] = {a.q0[n], a.q1[n], a.q2[n]};
   const double Et = a.E[n];
-  const double uv[3] = {qv[0] / rho, qv[1] / rho, qv[2] / rho};
-  const double umag = uv[0] * uv[0] + uv[1] * uv[1] + uv[2] * uv[2];
-  const double kk = 0.5 * umag;
-  const double p = rho * (g - 1.0) * ((Et / rho) - 0.5 * umag);
-  const double h = (g / (g - 1.0)) * p / rho;
-  const double T = p / (rho * Rg);
-  const double Ht = h + kk;
+  const double wm = a.w[n], we = a.w[n + 4 * N];
+  const double wmo[3] = {a.w[n + N], a.w[n + 2 * N], a.w[n + 3 * N]};
   const double mf = a.mu_factor[n];
-  const double muf = mf * kC1 * (T * sqrt(T)) / (T + kS);
-  const double dmuf_dT = mf * kC1 * (1.5 * sqrt(T) * (T + kS) - T * sqrt(T)) / ((T + kS) * (T + kS));
   const double mue = a.mue[(size_t)e * NN + d];
   const double musgs = a.musgs ? a.musgs[(size_t)e * NN + d] : 0.0;
+  double G[9];  // gpvol He
+  {
+    const double gpv = Ge[9 * NN + d];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) G[c] = gpv * Ge[c * NN + d];
+  }
+  const double irho = 1.0 / rho;
+  const double uv[3] = {qv[0] * irho, qv[1] * irho, qv[2] * irho};
+  const double kk = 0.5 * (uv[0] * uv[0] + uv[1] * uv[1] + uv[2] * uv[2]);
+  const double p = rho * (g - 1.0) * (Et * irho - kk);
+  const double h = a.prm.g_gm1 * p * irho;
+  const double T = p * irho * a.prm.inv_Rgas;
+  const double Ht = h + kk;
+  const double CpPr = a.prm.CpPr;
+  const double muf = mf * kC1 * (T * sqrt(T)) / (T + kS);
   // elem_diffu.f90: the molecular part of the stress carries rho mu_sgs (mu_fgp), the heat flux
   // Cp/0.9 rho mu_sgs; both enter the reverse sweep through rho
   const double mufgp = muf + rho * musgs;
-
-  // ---------------- forward recompute of the derivative quantities ----------------
-  double* Fw = sm;
-  Fw[F_RHO * FSTRIDE + s] = rho;
-  Fw[F_H * FSTRIDE + s] = Ht;
-  Fw[F_T * FSTRIDE + s] = T;
+  {
+    sm[F_RHO * FSTRIDE + s] = rho;
+    sm[F_H * FSTRIDE + s] = Ht;
+    sm[F_T * FSTRIDE + s] = T;
+    sm[W_M2 * FSTRIDE + s] = 2.0 * wm;
+    sm[W_E * FSTRIDE + s] = we;
+    sm[W_NU * FSTRIDE + s] = a.prm.c_rho * mue * irho * wm;
+    sm[W_KE * FSTRIDE + s] = (muf * CpPr + a.prm.c_ener * mue * CpPr + a.prm.Cp09 * rho * musgs) * we;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    Fw[(F_U0 + c) * FSTRIDE + s] = uv[c];
-    Fw[(F_Q0 + c) * FSTRIDE + s] = qv[c];
+    for (int c = 0; c < 3; ++c) {
+      sm[(F_U0 + c) * FSTRIDE + s] = uv[c];
+      sm[(W_O0 + c) * FSTRIDE + s] = wmo[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 9; ++c) sm[(F_G + c) * FSTRIDE + s] = G[c];
   }
   __syncthreads();
-  auto grad = [&](int f, double* o) {
-    double gx, gy, gz;
-    giso_line(Fw + f * FSTRIDE, i, j, k, Ds.d, gx, gy, gz);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) o[r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
-  };
-  double gRho[3], gH[3], gRH[3], gT[3], gU[3][3], gQ[3][3];
-  grad(F_RHO, gRho); grad(F_H, gH); grad(F_T, gT);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) { grad(F_U0 + c, gU[c]); grad(F_Q0 + c, gQ[c]); }
-  // the product fields rho H, H u_c and u (x) u are formed at the line points from the staged
-  // factors (the line weight applied to the first factor), not staged themselves
-  double divHu = 0.0, divFuu[3] = {0.0, 0.0, 0.0};
+  constexpr int stride[3] = {1, 4, PLANE};
+  const int line[3] = {sidx(0, j, k), sidx(i, 0, k), sidx(i, j, 0)};
+  const int row[3] = {i, j, k};
+
+  // ---------------- convection and pressure: both roles of every line pair ----------------
+  double rb = 0.0, Hb = 0.0, pb = 0.0;
+  double ub[3] = {0.0, 0.0, 0.0};
   {
-    double gRHi[3];
+    double X1 = 0.0, gb = 0.0;
 #pragma unroll
     for (int dir = 0; dir < 3; ++dir) {
-      double lRH = 0.0, lHu[3] = {0.0, 0.0, 0.0}, lUU[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      const int x = dir == 0 ? i : (dir == 1 ? j : k);
+      double w1[4], w2[4], Y1 = 0.0;
+      load4(dtab + 4 * row[dir], w1);
+      load4(dtab + 16 + 4 * row[dir], w2);
 #pragma unroll
       for (int m = 0; m < NP1; ++m) {
-        const int sp = dir == 0 ? sidx(m, j, k) : (dir == 1 ? sidx(i, m, k) : sidx(i, j, m));
-        const double w = Ds.d[x][m];
-        const double r_ = Fw[F_RHO * FSTRIDE + sp], H_ = Fw[F_H * FSTRIDE + sp];
-        const double u_[3] = {Fw[F_U0 * FSTRIDE + sp], Fw[F_U1 * FSTRIDE + sp], Fw[F_U2 * FSTRIDE + sp]};
-        const double wH = w * H_;
-        lRH += wH * r_;
+        const double* f = sm + line[dir] + m * stride[dir];
+        const double r_ = f[F_RHO * FSTRIDE], H_ = f[F_H * FSTRIDE];
+        const double br = rho + r_, bH = Ht + H_;
+        const double bu[3] = {uv[0] + f[F_U0 * FSTRIDE], uv[1] + f[F_U1 * FSTRIDE], uv[2] + f[F_U2 * FSTRIDE]};
+        const double gl[3] = {f[(F_G + dir) * FSTRIDE], f[(F_G + 3 + dir) * FSTRIDE], f[(F_G + 6 + dir) * FSTRIDE]};
+        const double el = f[W_E * FSTRIDE];
+        const double ol[3] = {f[W_O0 * FSTRIDE], f[W_O1 * FSTRIDE], f[W_O2 * FSTRIDE]};
+        const double bV1 = G[dir] * bu[0] + G[3 + dir] * bu[1] + G[6 + dir] * bu[2];
+        const double bV2 = gl[0] * bu[0] + gl[1] * bu[1] + gl[2] * bu[2];
+        double Q1 = 2.0 * wm + (wmo[0] * bu[0] + wmo[1] * bu[1] + wmo[2] * bu[2]);
+        double Q2 = f[W_M2 * FSTRIDE] + (ol[0] * bu[0] + ol[1] * bu[1] + ol[2] * bu[2]);
+        if constexpr (!TOTH) {
+          Q1 += we * bH;
+          Q2 += el * bH;
+        }
+        const double c1 = w1[m] * br, c2 = w2[m] * br;
+        const double P1 = w1[m] * bV1, P2 = w2[m] * bV2;
+        rb += P1 * Q1 + P2 * Q2;
+        const double x2 = c2 * bV2;
+        X1 += c1 * bV1;
+        double y2 = c2 * Q2;
+        if constexpr (TOTH) {
+          // the energy flux is (G_x + G_l)(V_x + V_l) / 2 with G = rho H
+          const double bg = rho * Ht + r_ * H_;
+          gb += P1 * we + P2 * el;
+          Y1 += c1 * Q1 + 2.0 * (w1[m] * bg) * we;
+          y2 += 2.0 * (w2[m] * bg) * el;
+        } else {
+          Hb += x2 * el;
+          Y1 += c1 * Q1;
+        }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) lHu[c] += wH * u_[c];
-        const double wu[3] = {w * u_[0], w * u_[1], w * u_[2]};
-#pragma unroll
-        for (int t = 0; t < 6; ++t) lUU[t] += wu[sym_c(t)] * u_[sym_j(t)];
+        for (int c = 0; c < 3; ++c) ub[c] += x2 * ol[c] + y2 * gl[c];
+        pb += w2[m] * (gl[0] * ol[0] + gl[1] * ol[1] + gl[2] * ol[2]);
       }
-      gRHi[dir] = lRH;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) divHu += H[3 * c + dir] * lHu[c];
-      // rows of the symmetric u (x) u: row0 = (00,01,02), row1 = (01,11,12), row2 = (02,12,22)
-      divFuu[0] += H[dir] * lUU[0] + H[3 + dir] * lUU[1] + H[6 + dir] * lUU[2];
-      divFuu[1] += H[dir] * lUU[1] + H[3 + dir] * lUU[3] + H[6 + dir] * lUU[4];
-      divFuu[2] += H[dir] * lUU[2] + H[3 + dir] * lUU[4] + H[6 + dir] * lUU[5];
+      for (int c = 0; c < 3; ++c) ub[c] += Y1 * G[3 * c + dir];
     }
 #pragma unroll
-    for (int r = 0; r < 3; ++r) gRH[r] = H[3 * r] * gRHi[0] + H[3 * r + 1] * gRHi[1] + H[3 * r + 2] * gRHi[2];
+    for (int c = 0; c < 3; ++c) ub[c] = 0.25 * (ub[c] + X1 * wmo[c]);
+    rb *= 0.25;
+    if constexpr (TOTH) {
+      rb += 0.5 * Ht * gb;
+      Hb = 0.5 * rho * gb;
+    } else {
+      Hb = 0.25 * (Hb + X1 * we);
+    }
   }
-  const double divU = gU[0][0] + gU[1][1] + gU[2][2];
-  const double divQ = gQ[0][0] + gQ[1][1] + gQ[2][2];
-  // diffusion pass 1 (stresses) and the contravariant gradRho / gradT fluxes for pass 2
-  const double mut = mufgp + mue;
-  double tau[3][3];
+
+  // ---------------- forward gradients, and D along the seed lines ----------------
+  pass_fence();
+  const double igpv = 1.0 / Ge[9 * NN + d];  // G holds gpvol He; the forward gradients want He
+  double gU[3][3];
+  {
+    double gRho[3] = {0.0, 0.0, 0.0}, gT[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) tau[r][c] = mut * (gU[r][c] + gU[c][r]);
+      for (int r = 0; r < 3; ++r) gU[c][r] = 0.0;
 #pragma unroll
-  for (int r = 0; r < 3; ++r) tau[r][r] -= mufgp * (2.0 / 3.0) * divU;
-  double* V6 = sm + NF_FWD * FSTRIDE;  // does not overlap the forward fields
+    for (int dir = 0; dir < 3; ++dir) {
+      double w1[4];
+      load4(dtab + 4 * row[dir], w1);
+      double lr = 0.0, lT = 0.0, lu[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int m = 0; m < NP1; ++m) {
+        const double* f = sm + line[dir] + m * stride[dir];
+        lr += w1[m] * f[F_RHO * FSTRIDE];
+        lT += w1[m] * f[F_T * FSTRIDE];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) lu[c] += w1[m] * f[(F_U0 + c) * FSTRIDE];
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const double hr = G[3 * r + dir];
+        gRho[r] += hr * lr;
+        gT[r] += hr * lT;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) gU[c][r] += hr * lu[c];
+      }
+    }
+    // contravariant grad rho and grad T fluxes (gpvol He^T grad) for the weak divergences below
+#pragma unroll
+    for (int dir = 0; dir < 3; ++dir) {
+      const double h0 = G[dir] * igpv, h1 = G[3 + dir] * igpv, h2 = G[6 + dir] * igpv;
+      sm[(F_V6 + dir) * FSTRIDE + s] = h0 * gRho[0] + h1 * gRho[1] + h2 * gRho[2];
+      sm[(F_V6 + 3 + dir) * FSTRIDE + s] = h0 * gT[0] + h1 * gT[1] + h2 * gT[2];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) gU[c][r] *= igpv;
+  }
+  pass_fence();
+  // adjoints of the contravariant fluxes (the adjoint of D^T is D along lines) back to the fluxes'
+  // physical components: Vb_r = gpvol He(r,:) . (D S_v)
+  double gRhob[3] = {0.0, 0.0, 0.0}, gTb[3] = {0.0, 0.0, 0.0}, tUb[3] = {0.0, 0.0, 0.0};
+  double taub[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
-    V6[dir * FSTRIDE + s] = gpv * (H[dir] * gRho[0] + H[3 + dir] * gRho[1] + H[6 + dir] * gRho[2]);
-    V6[(3 + dir) * FSTRIDE + s] = gpv * (H[dir] * gT[0] + H[3 + dir] * gT[1] + H[6 + dir] * gT[2]);
-  }
-  __syncthreads();  // forward fields consumed; V6 complete
-  const double divDr = divT_line(V6, V6 + FSTRIDE, V6 + 2 * FSTRIDE, i, j, k, Ds.d);
-  const double divDgT = divT_line(V6 + 3 * FSTRIDE, V6 + 4 * FSTRIDE, V6 + 5 * FSTRIDE, i, j, k, Ds.d);
-
-  // ---------------- reverse sweep ----------------
-  const int64_t N = a.npoin;
-  const double wm = a.w[n], we = a.w[n + 4 * N];
-  const double wmo[3] = {a.w[n + N], a.w[n + 2 * N], a.w[n + 3 * N]};
-  double rb = 0.0, Hb = 0.0, pb = 0.0, Tb = 0.0, mufb = 0.0;
-  double ub[3] = {0, 0, 0}, qb[3] = {0, 0, 0};
-  double gRhob[3] = {0, 0, 0}, gPb[3] = {0, 0, 0}, gHb[3] = {0, 0, 0}, gRHb[3] = {0, 0, 0}, gTb[3] = {0, 0, 0};
-  double gUb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, gQb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  double dFeb = 0.0, dFueb = 0.0, divUb = 0.0, divQb = 0.0;
-  double dFb[3] = {0, 0, 0}, dFuub[3] = {0, 0, 0};
-
-  // diffusion outputs (elem_diffu.f90:143-193): nu_e*divD(gradRho), divD(tauU) + kappa*divD(gradT),
-  // divD(tau row r); nu_e and kappa belong to the output node
-  const double CpPr = a.prm.Cp / a.prm.Prt;
-  const double nu_e = a.prm.c_rho * mue / rho;
-  const double kappa = muf * CpPr + a.prm.c_ener * mue * CpPr + a.prm.Cp09 * rho * musgs;
-  rb += wm * divDr * (-a.prm.c_rho * mue / (rho * rho));
-  mufb += we * divDgT * CpPr;
-  rb += we * divDgT * a.prm.Cp09 * musgs;
-  double* S6 = sm;  // overlaps forward fields only (read before the last barrier), not V6
-  S6[0 * FSTRIDE + s] = nu_e * wm;
-  S6[1 * FSTRIDE + s] = we;
-  S6[2 * FSTRIDE + s] = kappa * we;
+    double w1[4];
+    load4(dtab + 4 * row[dir], w1);
+    double l0 = 0.0, l1 = 0.0, l2 = 0.0, lo[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int r = 0; r < 3; ++r) S6[(3 + r) * FSTRIDE + s] = wmo[r];
-  __syncthreads();
-  {
-    double taub[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    for (int m = 0; m < NP1; ++m) {
+      const double* f = sm + line[dir] + m * stride[dir];
+      l0 += w1[m] * f[W_NU * FSTRIDE];
+      l1 += w1[m] * f[W_E * FSTRIDE];
+      l2 += w1[m] * f[W_KE * FSTRIDE];
 #pragma unroll
-    for (int v = 0; v < 6; ++v) {
-      double gx, gy, gz;
-      giso_line(S6 + v * FSTRIDE, i, j, k, Ds.d, gx, gy, gz);  // adjoint of D^T: D along lines
-      double Vb[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) Vb[r] = gpv * (H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz);
-      if (v == 0) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) gRhob[r] += Vb[r];
-      } else if (v == 1) {  // tauU_r = sum_c tau_rc u_c
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            taub[r][c] += Vb[r] * uv[c];
-            ub[c] += Vb[r] * tau[r][c];
-          }
-      } else if (v == 2) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) gTb[r] += Vb[r];
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) taub[v - 3][c] += Vb[c];
-      }
+      for (int c = 0; c < 3; ++c) lo[c] += w1[m] * f[(W_O0 + c) * FSTRIDE];
     }
-    // tau_rc = (mu_fgp+mue)(du_r/dx_c + du_c/dx_r) - delta_rc mu_fgp 2/3 div u, mu_fgp = muf + rho musgs
-    double mufgpb = 0.0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const double hr = G[3 * r + dir];
+      gRhob[r] += hr * l0;
+      tUb[r] += hr * l1;
+      gTb[r] += hr * l2;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) taub[c][r] += hr * lo[c];
+    }
+  }
+  // tauU_r = sum_c tau_rc u_c;  tau_rc = (mu_fgp+mue)(du_r/dx_c + du_c/dx_r) - delta_rc mu_fgp 2/3 div u,
+  // mu_fgp = muf + rho musgs
+  double Tb = 0.0;
+  double gUb[3][3];
+  {
+    const double divU = gU[0][0] + gU[1][1] + gU[2][2];
+    const double mut = mufgp + mue;
+    double mufgpb = 0.0, tr = 0.0;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        gUb[r][c] += mut * taub[r][c];
-        gUb[c][r] += mut * taub[r][c];
-        mufgpb += taub[r][c] * (gU[r][c] + gU[c][r]);
+        const double sg = gU[r][c] + gU[c][r];
+        double tau = mut * sg;
+        if (r == c) tau -= mufgp * (2.0 / 3.0) * divU;
+        ub[c] += tUb[r] * tau;
+        taub[r][c] += tUb[r] * uv[c];
+        mufgpb += taub[r][c] * sg;
       }
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      mufgpb += -taub[r][r] * (2.0 / 3.0) * divU;
-      divUb += -mufgp * (2.0 / 3.0) * taub[r][r];
-    }
-    mufb += mufgpb;
+    for (int r = 0; r < 3; ++r) tr += taub[r][r];
+    mufgpb -= (2.0 / 3.0) * divU * tr;
+    const double divUb = -mufgp * (2.0 / 3.0) * tr;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gUb[r][c] = mut * (taub[r][c] + taub[c][r]) + (r == c ? divUb : 0.0);
     rb += mufgpb * musgs;
+    Tb = mufgpb;  // d/d muf, finished below
   }
-
-  // convection (elem_convec.f90:412-434), seeds times gpvol; energy through H = h + k
+  __syncthreads();  // every line read of the first 22 arrays done; V6 complete
+  // nu_e and kappa belong to the output node (elem_diffu.f90:143-193)
   {
-    const double mm = gpv * wm, me = gpv * we;
-    const double mc[3] = {gpv * wmo[0], gpv * wmo[1], gpv * wmo[2]};
-    // mass: 1/2 (div q + rho div u + u . grad rho)
-    divQb += 0.5 * mm; rb += 0.5 * divU * mm; divUb += 0.5 * rho * mm;
+    double w2[3][4];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) { ub[c] += 0.5 * gRho[c] * mm; gRhob[c] += 0.5 * uv[c] * mm; }
-    if constexpr (TOTH) {
-      // full_convec_ijk_H (elem_convec.f90:171-177): 1/2 (div((E + p) u) + (E + p) div u
-      // + u.grad(E + p)) with E + p = rho H (the same function of rho, q, E)
-      dFeb += 0.5 * me;
-      rb += 0.5 * Ht * divU * me; Hb += 0.5 * rho * divU * me; divUb += 0.5 * rho * Ht * me;
+    for (int dir = 0; dir < 3; ++dir) load4(dtab + 16 + 4 * row[dir], w2[dir]);
+    double dr = 0.0, dT = 0.0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) { ub[c] += 0.5 * gRH[c] * me; gRHb[c] += 0.5 * uv[c] * me; }
-    } else {
-      // energy: 1/4 (H div q + rho H div u + q.grad H + u.grad(rho H) + H u.grad rho
-      //              + div(rho H u) + rho div(H u))
-      dFeb += 0.25 * me;
-      Hb += 0.25 * divQ * me; divQb += 0.25 * Ht * me;
-      rb += 0.25 * Ht * divU * me; Hb += 0.25 * rho * divU * me; divUb += 0.25 * rho * Ht * me;
-      rb += 0.25 * divHu * me; dFueb += 0.25 * rho * me;
+    for (int dir = 0; dir < 3; ++dir)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        qb[c] += 0.25 * gH[c] * me; gHb[c] += 0.25 * qv[c] * me;
-        ub[c] += 0.25 * gRH[c] * me; gRHb[c] += 0.25 * uv[c] * me;
-        Hb += 0.25 * uv[c] * gRho[c] * me; ub[c] += 0.25 * Ht * gRho[c] * me; gRhob[c] += 0.25 * Ht * uv[c] * me;
+      for (int m = 0; m < NP1; ++m) {
+        const double* f = sm + line[dir] + m * stride[dir];
+        dr += w2[dir][m] * f[(F_V6 + dir) * FSTRIDE];
+        dT += w2[dir][m] * f[(F_V6 + 3 + dir) * FSTRIDE];
       }
-    }
-    // momentum: 1/4 (div(q u) + u div q + q div u + rho div(u u) + u u.grad rho + q.grad u + u.grad q)
-    //           + grad p
+    rb += wm * dr * (-a.prm.c_rho * mue * irho * irho) + we * dT * a.prm.Cp09 * musgs;
+    Tb += we * dT * CpPr;
+    // gradient adjoints -> iso adjoints (He^T) on the arrays the passes above no longer read
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double mu_c = mc[c];
-      dFb[c] += 0.25 * mu_c;
-      ub[c] += 0.25 * divQ * mu_c; divQb += 0.25 * uv[c] * mu_c;
-      qb[c] += 0.25 * divU * mu_c; divUb += 0.25 * qv[c] * mu_c;
-      rb += 0.25 * divFuu[c] * mu_c; dFuub[c] += 0.25 * rho * mu_c;
-      gPb[c] += mu_c;
-#pragma unroll
-      for (int jd = 0; jd < 3; ++jd) {
-        ub[c] += 0.25 * uv[jd] * gRho[jd] * mu_c;
-        ub[jd] += 0.25 * uv[c] * gRho[jd] * mu_c;
-        gRhob[jd] += 0.25 * uv[c] * uv[jd] * mu_c;
-        qb[jd] += 0.25 * gU[c][jd] * mu_c;
-        gUb[c][jd] += 0.25 * qv[jd] * mu_c;
-        ub[jd] += 0.25 * gQ[c][jd] * mu_c;
-        gQb[c][jd] += 0.25 * uv[jd] * mu_c;
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      gUb[c][c] += divUb;
-      gQb[c][c] += divQb;
-    }
-  }
-
-  // derivative adjoints -> iso adjoints (He^T) -> D^T line sums, in chunks of kChunk fields
-  auto iso3 = [&](int f, double* o) {
-    if (f <= A_Q2) {  // gradient fields: sum_r He(r,dir) gb_r
-      const double* gb = f == A_RHO ? gRhob : f == A_P ? gPb : f == A_H ? gHb : f == A_RH ? gRHb
-                         : f == A_T ? gTb : f <= A_U2 ? gUb[f - A_U0] : gQb[f - A_Q0];
-#pragma unroll
-      for (int dir = 0; dir < 3; ++dir) o[dir] = H[dir] * gb[0] + H[3 + dir] * gb[1] + H[6 + dir] * gb[2];
-    } else if (f <= A_FUE2) {  // component c of a vector whose divergence has adjoint db
-      const int c = f <= A_FE2 ? f - A_FE0 : f - A_FUE0;
-      const double db = f <= A_FE2 ? dFeb : dFueb;
-#pragma unroll
-      for (int dir = 0; dir < 3; ++dir) o[dir] = H[3 * c + dir] * db;
-    } else {  // symmetric (c,jj) entry: row c takes d/dx_jj, row jj takes d/dx_c
-      const int t = f <= A_F22 ? f - A_F00 : f - A_UU00;
-      const double* db = f <= A_F22 ? dFb : dFuub;
-      const int c = sym_c(t), jj = sym_j(t);
-#pragma unroll
-      for (int dir = 0; dir < 3; ++dir)
-        o[dir] = H[3 * jj + dir] * db[c] + (c != jj ? H[3 * c + dir] * db[jj] : 0.0);
-    }
-  };
-  // nodal product fields -> primitives (product rule at the output node)
-  auto apply = [&](int f, double t) {
-    if (f == A_RHO) {
-      rb += t;
-    } else if (f == A_P) {
-      pb += t;
-    } else if (f == A_H) {
-      Hb += t;
-    } else if (f == A_RH) {
-      rb += Ht * t; Hb += rho * t;
-    } else if (f == A_T) {
-      Tb += t;
-    } else if (f <= A_U2) {
-      ub[f - A_U0] += t;
-    } else if (f <= A_Q2) {
-      qb[f - A_Q0] += t;
-    } else if (f <= A_FE2) {  // rho H u_c
-      const int c = f - A_FE0;
-      rb += Ht * uv[c] * t; Hb += rho * uv[c] * t; ub[c] += rho * Ht * t;
-    } else if (f <= A_FUE2) {  // H u_c
-      const int c = f - A_FUE0;
-      Hb += uv[c] * t; ub[c] += Ht * t;
-    } else if (f <= A_F22) {  // q_c u_jj
-      const int c = sym_c(f - A_F00), jj = sym_j(f - A_F00);
-      qb[c] += uv[jj] * t; ub[jj] += qv[c] * t;
-    } else {  // u_c u_jj
-      const int c = sym_c(f - A_UU00), jj = sym_j(f - A_UU00);
-      ub[c] += uv[jj] * t; ub[jj] += uv[c] * t;
-    }
-  };
-  __syncthreads();  // seed arrays consumed before the chunks overwrite them
-#pragma unroll
-  for (int c0 = 0; c0 < NF_ADJ; c0 += kChunk) {
-#pragma unroll
-    for (int f = c0; f < c0 + kChunk && f < NF_ADJ; ++f) {
-      double o[3];
-      iso3(f, o);
-#pragma unroll
-      for (int dir = 0; dir < 3; ++dir) sm[((f - c0) * 3 + dir) * FSTRIDE + s] = o[dir];
+    for (int dir = 0; dir < 3; ++dir) {
+      const double h0 = G[dir] * igpv, h1 = G[3 + dir] * igpv, h2 = G[6 + dir] * igpv;
+      auto put = [&](int f, const double* gb) { sm[(3 * f + dir) * FSTRIDE + s] = h0 * gb[0] + h1 * gb[1] + h2 * gb[2]; };
+      put(0, gUb[0]);
+      put(1, gUb[1]);
+      put(2, gUb[2]);
+      put(3, gRhob);
+      put(4, gTb);
     }
     __syncthreads();
+    double lT = 0.0;
 #pragma unroll
-    for (int f = c0; f < c0 + kChunk && f < NF_ADJ; ++f) {
-      const double* b = sm + (size_t)(f - c0) * 3 * FSTRIDE;
-      apply(f, divT_line(b, b + FSTRIDE, b + 2 * FSTRIDE, i, j, k, Ds.d));
-    }
-    if (c0 + kChunk < NF_ADJ) __syncthreads();
+    for (int dir = 0; dir < 3; ++dir)
+#pragma unroll
+      for (int m = 0; m < NP1; ++m) {
+        const double* f = sm + line[dir] + m * stride[dir];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ub[c] += w2[dir][m] * f[(3 * c + dir) * FSTRIDE];
+        rb += w2[dir][m] * f[(9 + dir) * FSTRIDE];
+        lT += w2[dir][m] * f[(12 + dir) * FSTRIDE];
+      }
+    // Sutherland (mod_fluid_viscosity.f90:37)
+    const double dmuf_dT = mf * kC1 * (1.5 * sqrt(T) * (T + kS) - T * sqrt(T)) / ((T + kS) * (T + kS));
+    Tb = Tb * dmuf_dT + lT;
   }
 
-  // H = h + k; Sutherland, EOS and u = q/rho in reverse (time_integ.f90:266-285,
-  // mod_fluid_viscosity.f90:37)
-  double hb = Hb, kb = Hb;
-  Tb += mufb * dmuf_dT;
-  pb += hb * g / ((g - 1.0) * rho);
-  rb += -hb * h / rho;
-  pb += Tb / (rho * Rg);
-  rb += -Tb * T / rho;
+  // H = h + k, EOS and u = q/rho in reverse (time_integ.f90:266-285)
+  double kb = Hb;
+  pb += Hb * a.prm.g_gm1 * irho;
+  rb += -Hb * h * irho;
+  pb += Tb * irho * a.prm.inv_Rgas;
+  rb += -Tb * T * irho;
   const double Eb = (g - 1.0) * pb;
   rb += -(g - 1.0) * kk * pb;
   kb += -(g - 1.0) * rho * pb;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) ub[c] += uv[c] * kb;
+  double qb[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    qb[c] += ub[c] / rho;
-    rb += -uv[c] * ub[c] / rho;
+    ub[c] += uv[c] * kb;
+    qb[c] = ub[c] * irho;
+    rb += -uv[c] * qb[c];
   }
   store_res6<double>(a.out, (size_t)e * NN + d, rb, qb[0], qb[1], qb[2], Eb, 0.0);
 }
