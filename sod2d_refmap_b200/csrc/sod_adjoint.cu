@@ -673,7 +673,7 @@ int sod_rk4_step_vjp(SodMesh* m, const double* rho, const double* q, const doubl
     for (int t = 0; t < 3; ++t) ys[t] = stages + (size_t)t * 5 * N;
   } else {
     // forward recompute of the stage states (mu_e and dt frozen)
-    const int epb = m->tuned_epb[0] ? m->tuned_epb[0] : 2;
+    const int epb = rhs_epb(m, false);
     const double acoef[3] = {0.5, 0.5, 1.0};
     Cols5 cur = Y1;
     for (int t = 0; t < 3; ++t) {
@@ -704,7 +704,7 @@ int sod_rk4_step_vjp(SodMesh* m, const double* rho, const double* q, const doubl
     }
   }
   if (ff || slip) {
-    const int epb = m->tuned_epb[0] ? m->tuned_epb[0] : 2;
+    const int epb = rhs_epb(m, false);
     if ((slip || ffz) && stages) {
       // the stage residuals at the slip nodes / lnbn targets (the recompute gathered them already)
       for (int t = 0; t < 3; ++t) {

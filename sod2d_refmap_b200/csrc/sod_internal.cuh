@@ -329,6 +329,10 @@ int launch_copy_f32(const double* src, float* dst, int64_t n, cudaStream_t st);
 int init_kernel_attrs();
 // bounded host wait (sod_set_wait_timeout) and the non-finite flag of the stage-4 gather
 constexpr int kNonfiniteCounter = 1;  // index in StepBuffers::counters
+// Elements per CTA of the fused RHS when neither sod_autotune nor sod_set_rhs_config chose: one.  At
+// 64^3 one / two / four take 0.826 / 0.840 / 1.042 ms mixed and 0.986 / 1.048 / 1.160 ms FP64 (two
+// elements wait at each other's barriers), and at 8^3 one spreads 512 CTAs over all SMs.
+inline int rhs_epb(const SodMesh* m, bool mixed) { return m->tuned_epb[mixed ? 1 : 0] ? m->tuned_epb[mixed ? 1 : 0] : 1; }
 int sync_stream(cudaStream_t st);
 int take_nonfinite(SodMesh* m, cudaStream_t st, bool* flagged);
 // boundary conditions (sod_bc.cu), used by the step pipeline when m->bc.nb > 0

@@ -628,7 +628,7 @@ int run_step(SodMesh* m, SodState* s, const double* dt_dev, double* dt_next, boo
              cudaEvent_t* ev = nullptr, double* stage_store = nullptr, cudaEvent_t state_done = nullptr) {
   NvtxRange range(mixed ? "sod rk4 step (mixed)" : "sod rk4 step (fp64)");
   const size_t N = m->npoin;
-  const int epb = m->tuned_epb[mixed ? 1 : 0] ? m->tuned_epb[mixed ? 1 : 0] : (mixed ? 4 : 2);
+  const int epb = rhs_epb(m, mixed);
   SodState loc = *s;
   const bool les = les_active(m, s);
   double* reta_tmp = nullptr;
@@ -1075,7 +1075,7 @@ int sod_rhs(SodMesh* m, const double* rho, const double* q, const double* E, con
     if (rc) return rc;
   }
   const size_t N = m->npoin;
-  const int epb = m->tuned_epb[mixed ? 1 : 0] ? m->tuned_epb[mixed ? 1 : 0] : (mixed ? 4 : 2);
+  const int epb = rhs_epb(m, mixed);
   rc = launch_rhs(m, mixed, epb, rho, q, q + N, q + 2 * N, E, mu_factor, nullptr, st);
   if (rc) return rc;
   GatherArgs g{};
