@@ -65,11 +65,13 @@ void sod_batch_destroy(SodBatch* B) {
   if (B->ref_mue) cudaFree(B->ref_mue);
   if (B->mesh) {
     SodMesh* m = B->mesh;
-    void* ptrs[] = {m->node_member, m->elem_member, m->member_node_off, m->member_scal, m->member_dt_bits};
+    void* ptrs[] = {m->node_member, m->elem_member, m->member_node_off, m->member_scal, m->member_dt_bits, m->member_red,
+                    m->member_done};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     m->node_member = m->elem_member = m->member_node_off = nullptr;
-    m->member_scal = m->member_dt_bits = nullptr;
+    m->member_scal = m->member_dt_bits = m->member_red = nullptr;
+    m->member_done = nullptr;
     sod_mesh_destroy(m);
   }
   delete B;
@@ -151,6 +153,8 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
   BALLOC(m->member_node_off, sizeof(int32_t) * (nmesh + 1));
   BALLOC(m->member_scal, sizeof(double) * 2 * nmesh);
   BALLOC(m->member_dt_bits, sizeof(double) * nmesh);
+  BALLOC(m->member_red, sizeof(double) * 3 * kEtaChunks * nmesh);
+  BALLOC(m->member_done, sizeof(unsigned int) * nmesh);
   BALLOC(B->dt, sizeof(double) * nmesh);
   BALLOC(B->ref_mue, sizeof(double) * E * NN);
   {
@@ -164,6 +168,7 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
 #undef BALLOC
   cudaMemcpy(m->a_of_d_dev, m0->a_of_d_dev, sizeof(int32_t) * NN, cudaMemcpyDeviceToDevice);
   cudaMemset(m->mue_int, 0, sizeof(double) * E * NN);
+  cudaMemset(m->member_done, 0, sizeof(unsigned int) * nmesh);
   cudaMemset(B->st.mu_e, 0, sizeof(double) * E * NN);
   cudaMemcpy(m->member_node_off, B->node_off.data(), sizeof(int32_t) * (nmesh + 1), cudaMemcpyHostToDevice);
   int64_t nnz_off = 0;

@@ -27,6 +27,7 @@ constexpr int P = 3;
 constexpr int NP1 = P + 1;
 constexpr int NN = NP1 * NP1 * NP1;   // 64 nodes / gauss points per element
 constexpr int NGEO = 10;              // 9 He entries + gpvol
+constexpr int kEtaChunks = 32;        // blocks per ensemble member of the entropy statistics
 constexpr int NRES = 6;               // element residual fields: mass, mom x3, ener, eta
 constexpr double kSuthC1 = 0.000001458;  // sutherland_viscosity (mod_fluid_viscosity.f90:21-41)
 constexpr double kSuthS = 110.4;
@@ -296,6 +297,8 @@ struct SodMesh {
   int32_t* member_node_off = nullptr;  // [nmember+1] contiguous node ranges
   double* member_scal = nullptr;    // [nmember][2] eta mean, eta norm
   double* member_dt_bits = nullptr; // [nmember] scratch for the per-member dt min
+  double* member_red = nullptr;     // [nmember][kEtaChunks][3] partial entropy sums
+  unsigned int* member_done = nullptr;  // [nmember] chunks finished (zero between launches)
   double* musgs_int = nullptr;  // LES: internal-layout SGS viscosity (FP64), allocated on first use
   // adjoint scratch (sod_adjoint.cu): stage states, seeds, accumulators
   double* adj = nullptr;
