@@ -5,7 +5,13 @@
 // alpha = |grad u|^2 and beta = hLES^2 grad u^T grad u, the point value is
 // c_sgs sqrt(max(B(beta), 1e-10) / alpha) where alpha > 1e-10 (B = sum of the principal 2x2
 // minors), else the previous mu_sgs; the 3x3x3 convertIJK filter of the entropy viscosity then
-// smooths it inside the element.  Element-local, so the update of musgs_int is in place.
+// smooths it inside the element, as three 3-point passes (weights and index map are separable).
+// Element-local, so the update of musgs_int is in place.
+//
+// Bounded by memory latency on its inputs (10 metric values, 3 gathered velocities and the old value
+// per point).  D comes from a shared table (indexed by lane in the kernel parameters it was copied to
+// local memory: 128 bytes of stack, and a chain of local loads under every sum), and the lane order
+// is the RHS kernels': 24^3 elements 41 -> 28 us.
 #include "sod_internal.cuh"
 
 namespace sod {
@@ -20,38 +26,45 @@ __device__ __forceinline__ int nb_filter(int x) {  // natural index of convertIJ
 __global__ void __launch_bounds__(64 * EPB) k_sgs(int nelem, const int32_t* __restrict__ econn,
                                                  const double* __restrict__ geo, const double* __restrict__ u0,
                                                  const double* __restrict__ u1, const double* __restrict__ u2,
-                                                 const DMat D, double c_sgs, double* __restrict__ musgs) {
+                                                 const __grid_constant__ DMat D, double c_sgs,
+                                                 double* __restrict__ musgs) {
   __shared__ double us[EPB][3][FSTRIDE];
-  __shared__ double ml[EPB][NN];
-  const int es = threadIdx.x >> 6, d = threadIdx.x & 63;
+  __shared__ double ml[EPB][2][NN];
+  __shared__ __align__(16) double Ds[NP1 * NP1];
+  const int es = threadIdx.x >> 6, lt = threadIdx.x & 63;
   const int e = blockIdx.x * EPB + es;
   const bool act = e < nelem;
   const int ee = act ? e : nelem - 1;
-  const int i = d & 3, j = (d >> 2) & 3, k = d >> 4, s = sidx(i, j, k);
+  // lane bits (i0 j0 i1 j1 k): one shared-memory wavefront per xi and eta line load
+  const int i = (lt & 1) | ((lt >> 1) & 2), j = ((lt >> 1) & 1) | ((lt >> 2) & 2), k = lt >> 4;
+  const int d = i + 4 * j + 16 * k, s = sidx(i, j, k);
   const int n = econn[(size_t)ee * NN + d];
-  us[es][0][s] = u0[n];
-  us[es][1][s] = u1[n];
-  us[es][2][s] = u2[n];
   const double* G = geo + (size_t)ee * NGEO * NN;
   double H[9];
 #pragma unroll
   for (int c = 0; c < 9; ++c) H[c] = G[c * NN + d];
   const double gpv = G[9 * NN + d];
   const double old = musgs[(size_t)ee * NN + d];
+  if (threadIdx.x < NP1 * NP1) Ds[threadIdx.x] = D.d[threadIdx.x >> 2][threadIdx.x & 3];
+  us[es][0][s] = u0[n];
+  us[es][1][s] = u1[n];
+  us[es][2][s] = u2[n];
   __syncthreads();
   double gu[3][3];  // gu[c][r] = d u_c / d x_r
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const double* f = us[es][c];
-    double gx = 0.0, gy = 0.0, gz = 0.0;
+  for (int dir = 0; dir < 3; ++dir) {
+    const double* f = &us[es][0][0] + (dir == 0 ? sidx(0, j, k) : (dir == 1 ? sidx(i, 0, k) : sidx(i, j, 0)));
+    const int st = dir == 0 ? 1 : (dir == 1 ? 4 : PLANE);
+    const double* w = Ds + 4 * (dir == 0 ? i : (dir == 1 ? j : k));
+    double l[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int m = 0; m < NP1; ++m) {
-      gx += D.d[i][m] * f[sidx(m, j, k)];
-      gy += D.d[j][m] * f[sidx(i, m, k)];
-      gz += D.d[k][m] * f[sidx(i, j, m)];
-    }
+    for (int m = 0; m < NP1; ++m)
 #pragma unroll
-    for (int r = 0; r < 3; ++r) gu[c][r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
+      for (int c = 0; c < 3; ++c) l[c] += w[m] * f[c * FSTRIDE + m * st];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) gu[c][r] = dir == 0 ? H[3 * r] * l[c] : gu[c][r] + H[3 * r + dir] * l[c];
   }
   const double hLES = cbrt(gpv);
   double alpha = 0.0, V[3][3];
@@ -64,19 +77,17 @@ __global__ void __launch_bounds__(64 * EPB) k_sgs(int nelem, const int32_t* __re
     }
   const double B = V[0][0] * V[1][1] + V[0][0] * V[2][2] + V[1][1] * V[2][2] - V[0][1] * V[0][1] -
                    V[0][2] * V[0][2] - V[1][2] * V[1][2];
-  ml[es][d] = alpha > 1.0e-10 ? c_sgs * sqrt(fmax(B, 1.0e-10) / alpha) : old;
+  double* m0 = ml[es][0];
+  double* m1 = ml[es][1];
+  m0[d] = alpha > 1.0e-10 ? c_sgs * sqrt(fmax(B, 1.0e-10) / alpha) : old;
   __syncthreads();
-  const int ix[3] = {nb_filter(i - 1), i, nb_filter(i + 1)};
-  const int jx[3] = {nb_filter(j - 1), j, nb_filter(j + 1)};
-  const int kx[3] = {nb_filter(k - 1), k, nb_filter(k + 1)};
-  const double w[3] = {0.25, 0.5, 0.25};
-  double acc = 0.0;
-#pragma unroll
-  for (int l = 0; l < 3; ++l)
-#pragma unroll
-    for (int mm = 0; mm < 3; ++mm)
-#pragma unroll
-      for (int nn = 0; nn < 3; ++nn) acc = acc + w[l] * w[mm] * w[nn] * ml[es][ix[l] + 4 * jx[mm] + 16 * kx[nn]];
+  m1[d] = 0.25 * m0[nb_filter(i - 1) + 4 * j + 16 * k] + 0.5 * m0[d] + 0.25 * m0[nb_filter(i + 1) + 4 * j + 16 * k];
+  __syncthreads();
+  // m0 was last read before the barrier above
+  m0[d] = 0.25 * m1[i + 4 * nb_filter(j - 1) + 16 * k] + 0.5 * m1[d] + 0.25 * m1[i + 4 * nb_filter(j + 1) + 16 * k];
+  __syncthreads();
+  const double acc =
+      0.25 * m0[i + 4 * j + 16 * nb_filter(k - 1)] + 0.5 * m0[d] + 0.25 * m0[i + 4 * j + 16 * nb_filter(k + 1)];
   if (act) musgs[(size_t)e * NN + d] = acc;
 }
 
