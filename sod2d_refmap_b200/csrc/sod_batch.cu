@@ -269,12 +269,8 @@ int sod_batch_rk4_steps(SodBatch* B, int nsteps, SodPrecision prec, sod_stream_t
   const bool mixed = prec == SOD_MIXED;
   int rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, B->st.mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, B->st.mu_e, mixed, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   if (nsteps > 0) {
     const uint64_t key = ((uint64_t)mixed << 40) ^ ((uint64_t)m->persist_ctas[mixed ? 1 : 0] << 16) ^
                          (uint64_t)m->tuned_epb[mixed ? 1 : 0];

@@ -325,8 +325,11 @@ int mesh_from_device_ref(int nelem, int npoin, int base, const int32_t* connec, 
                          const int32_t* gI, const int32_t* gJ, const int32_t* gK, const double* wgp,
                          const double* helem_l, const double* helem, int npoin_w, const int32_t* lpoin_w,
                          const SodParams* params, cudaStream_t st, SodMesh** out);
+// f32_copy (optional): FP32 copy of the internal array
 int mesh_ref_to_internal_elem(SodMesh* m, const double* ref_dev /*(nelem,64) F*/, double* int_dev,
-                              cudaStream_t st);
+                              cudaStream_t st, float* f32_copy = nullptr);
+// the caller's mu_e into mue_int and, on the mixed path, mue32
+int mesh_mue_in(SodMesh* m, const double* mu_e, bool mixed, cudaStream_t st);
 int mesh_internal_to_ref_elem(SodMesh* m, const double* int_dev, double* ref_dev, cudaStream_t st);
 int launch_copy_f32(const double* src, float* dst, int64_t n, cudaStream_t st);
 int init_kernel_attrs();

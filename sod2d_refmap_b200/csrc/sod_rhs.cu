@@ -776,14 +776,10 @@ static int rk4_main_impl(SodMesh* m, SodState* s, const double* dt_dev, double* 
   const bool mixed = prec == SOD_MIXED;
   rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, s->mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, s->mu_e, mixed, st);
   if (rc) return rc;
   rc = les_in(m, s, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   rc = run_step(m, s, dt_dev, dt_next_dev, mixed, st, nullptr, nullptr, state_done);
   if (rc) return rc;
   rc = les_out(m, s, st);
@@ -801,14 +797,10 @@ int sod_rk4_main_record(SodMesh* m, SodState* s, const double* dt_dev, double* d
   const bool mixed = prec == SOD_MIXED;
   rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, s->mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, s->mu_e, mixed, st);
   if (rc) return rc;
   rc = les_in(m, s, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   rc = run_step(m, s, dt_dev, dt_next_dev, mixed, st, nullptr, stages);
   if (rc) return rc;
   rc = les_out(m, s, st);
@@ -825,14 +817,10 @@ int sod_rk4_steps(SodMesh* m, SodState* s, double* dt_dev, int nsteps, SodPrecis
   const bool mixed = prec == SOD_MIXED;
   rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, s->mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, s->mu_e, mixed, st);
   if (rc) return rc;
   rc = les_in(m, s, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   if (nsteps > 0) {
     // capture one step into a graph keyed by (state pointers, dt pointer, precision, epb)
     uint64_t key = (uint64_t)(uintptr_t)s->rho ^ ((uint64_t)(uintptr_t)dt_dev << 1) ^ ((uint64_t)mixed << 63) ^
@@ -884,14 +872,10 @@ int sod_step_profile(SodMesh* m, SodState* s, double* dt_dev, int nsteps, SodPre
   const bool mixed = prec == SOD_MIXED;
   rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, s->mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, s->mu_e, mixed, st);
   if (rc) return rc;
   rc = les_in(m, s, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   cudaEvent_t ev[18];
   for (int q = 0; q < 18; ++q) SOD_CUDA(cudaEventCreate(&ev[q]));
   double acc[3] = {0, 0, 0};
@@ -969,14 +953,10 @@ int sod_autotune(SodMesh* m, SodState* s, SodPrecision prec, int* best_epb, floa
   const bool mixed = prec == SOD_MIXED;
   rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, s->mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, s->mu_e, mixed, st);
   if (rc) return rc;
   rc = les_in(m, s, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   const size_t N = m->npoin;
   const int cand[] = {1, 2, 4, 8};
   cudaEvent_t e0, e1;
@@ -1087,12 +1067,8 @@ int sod_rhs(SodMesh* m, const double* rho, const double* q, const double* E, con
   const bool mixed = prec == SOD_MIXED;
   int rc = ensure_step_buffers(m, mixed);
   if (rc) return rc;
-  rc = mesh_ref_to_internal_elem(m, mu_e, m->mue_int, st);
+  rc = mesh_mue_in(m, mu_e, mixed, st);
   if (rc) return rc;
-  if (mixed) {
-    rc = launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st);
-    if (rc) return rc;
-  }
   const size_t N = m->npoin;
   const int epb = rhs_epb(m, mixed);
   rc = launch_rhs(m, mixed, epb, rho, q, q + N, q + 2 * N, E, mu_factor, nullptr, st);
