@@ -475,9 +475,9 @@ __global__ void __launch_bounds__(256) k_stage_state(int64_t N, const int32_t* _
 #pragma unroll
     for (int d = 0; d < 3; ++d) r[1 + d] += wmc[d * N + n];
   }
-  const double da = (*dt) * coef;
+  const double da = (*dt) * coef, iml = 1.0 / ml;
 #pragma unroll
-  for (int f = 0; f < 5; ++f) ys[f * N + n] = y.c[f][n] - da * (r[f] / ml);
+  for (int f = 0; f < 5; ++f) ys[f * N + n] = y.c[f][n] - da * (r[f] * iml);
 }
 
 // y0 - dt sum_s b_s R_s from the stage states (dt R_1 = 2 (y0 - Y2), dt R_2 = 2 (y0 - Y3),

@@ -254,6 +254,11 @@ int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStr
   return SOD_OK;
 }
 
+__global__ void k_inverse(int64_t n, const double* __restrict__ v, double* __restrict__ out) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) out[t] = v[t] != 0.0 ? 1.0 / v[t] : 0.0;
+}
+
 // Local node order of the library (natural d = i + 4j + 16k) from the reference's gmshAtoI/J/K
 // maps (host arrays, index_base-based), the 1-D derivative matrix from dlxigp_ip and, when given,
 // the GLL weights in that order.
@@ -300,6 +305,15 @@ int ensure_step_buffers(SodMesh* m, bool mixed) {
     SOD_CUDA(cudaMemset(b.counters, 0, sizeof(unsigned int) * 16));
     SOD_CUDA(cudaMalloc(&b.mu_fluid, sizeof(double) * N));
   }
+  bool filled = false;  // by kernels on the default stream, which the caller's stream may not wait for
+  if (!b.iml && m->Ml) {  // (a mesh view of the sod_*_ref entries has no lumped mass and no step)
+    double* v = nullptr;
+    SOD_CUDA(cudaMalloc(&v, sizeof(double) * N));
+    b.iml = v;
+    k_inverse<<<(unsigned)((N + 255) / 256), 256>>>(N, m->Ml, v);
+    SOD_CHECK_LAUNCH();
+    filled = true;
+  }
   size_t need = (size_t)E * NRES * NN * sizeof(double);  // sized for FP64 (also holds FP32)
   if (b.rel_bytes < need) {
     if (b.rel) cudaFree(b.rel);
@@ -311,12 +325,15 @@ int ensure_step_buffers(SodMesh* m, bool mixed) {
       SOD_CUDA(cudaMalloc(&m->geo32, sizeof(float) * E * NGEO * NN));
       int rc = launch_copy_f32(m->geo64, m->geo32, E * NGEO * NN, 0);
       if (rc) return rc;
+      filled = true;
     }
     if (!m->mue32) {
       SOD_CUDA(cudaMalloc(&m->mue32, sizeof(float) * E * NN));
       SOD_CUDA(cudaMemset(m->mue32, 0, sizeof(float) * E * NN));
+      filled = true;
     }
   }
+  if (filled) SOD_CUDA(cudaStreamSynchronize(0));
   return SOD_OK;
 }
 
@@ -402,7 +419,7 @@ void sod_mesh_destroy(SodMesh* m) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   void* ptrs[] = {m->econn, m->geo64, m->geo32, m->Ml, m->helem, m->helem_l, m->jratio, m->n2e_ptr, m->n2e,
                   m->mue_int, m->mue32, m->a_of_d_dev, m->buf.ys, m->buf.rsum, m->buf.rel, m->buf.red,
-                  m->buf.scal, m->buf.counters, m->buf.mu_fluid, m->adj, m->musgs_int};
+                  m->buf.scal, m->buf.counters, m->buf.mu_fluid, m->buf.iml, m->adj, m->musgs_int};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (double* p : m->host_mirror) cudaFree(p);

@@ -267,13 +267,13 @@ __global__ void __launch_bounds__(64 * EPB) k_stage_fused(const StageArgs p) {
 // resident 256-thread blocks per SM the register budget must allow.  FP32 residual rows (mixed
 // path): 4 blocks, 64 registers, no spill with the predicated groups of 4, 2% faster than full
 // groups at 5 blocks (the predicated groups at 5 blocks spilled 76 bytes and ran 4% slower
-// than that).  FP64 rows: 5 blocks, 48 registers (48-72 bytes of spill), 1% faster than 4
-// blocks; 7 blocks capped the kernel at 32 registers and spilled 140-244 bytes
+// than that).  FP64 rows: bounded for 3 blocks the kernel takes 56-64 registers without spill, so 4
+// still fit; bounded for 4 it spills 16 bytes, for 5 (48 registers) 76
 #ifndef SOD_KG_MIN_BLOCKS
 #define SOD_KG_MIN_BLOCKS 4
 #endif
 #ifndef SOD_KG_MIN_BLOCKS_F64
-#define SOD_KG_MIN_BLOCKS_F64 5
+#define SOD_KG_MIN_BLOCKS_F64 3
 #endif
 template <typename R, int STAGE>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? SOD_KG_MIN_BLOCKS : SOD_KG_MIN_BLOCKS_F64) k_gather_rk(const GatherArgs a) {
@@ -471,8 +471,10 @@ static void fill_gather_args(SodMesh* m, int stage, GatherArgs& a) {
   a.idx = m->n2e;
   a.rel = m->buf.rel;
   a.Ml = m->Ml;
+  a.iml = m->buf.iml;
   a.gamma = m->prm.gamma;
-  a.Rgas = m->prm.Rgas;
+  a.inv_Rgas = m->prm.inv_Rgas;
+  a.inv_gm1 = m->prm.inv_gm1;
   a.normalise = m->prm.normalise;
   if (!a.ys) a.ys = m->buf.ys;
   a.rsum = m->buf.rsum;

@@ -19,6 +19,7 @@ struct GatherArgs {
   const int32_t* __restrict__ idx;
   const void* rel;
   const double* __restrict__ Ml;
+  const double* __restrict__ iml;  // 1 / Ml, formed once with the step buffers
   const double* __restrict__ dt;  // device scalar, or per-member array when node_member is set
   const int32_t* __restrict__ node_member;
   int member_reduce;              // stage 4: eta sums done by the per-member kernel instead
@@ -33,7 +34,7 @@ struct GatherArgs {
   // stage-4 EOS outputs
   double *u0, *u1, *u2, *pr, *Tem, *e_int, *eta, *csound, *machno, *mu_fluid, *Reta;
   const double* mu_factor;
-  double gamma, Rgas;
+  double gamma, inv_Rgas, inv_gm1;  // 1/Rgas, 1/(gamma-1)
   double* red;              // partials [3*nblocks]
   unsigned int* counter;
   unsigned int* nonfinite;  // raised by stage 4 on a NaN/Inf in the new rho, q, E
@@ -94,49 +95,14 @@ __device__ __forceinline__ bool gather_rk_node(const GatherArgs& a, int n, doubl
 #pragma unroll
       for (int f = 0; f < 6; ++f) rsv[f] = STAGE == 1 ? (R)0 : rsum[f * N + n];
     }
-    const double ml = a.Ml[n];
+    const double iml = a.iml[n];  // 1 / Ml
     double r[6] = {0, 0, 0, 0, 0, 0};
     const int beg = a.ptr[n], end = a.ptr[n + 1];
-    int c = beg;
-    if constexpr (sizeof(R) == 4) {
-      // groups of up to 4 contributions (a partial group's missing ones predicated off): all
-      // loads of a group issued before its (ascending, fixed-order) sums, so a node with 1-4
-      // contributions waits on one chain of index -> residual loads
-      for (; c < end; c += 4) {
-        R v[4][6];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (c + q < end) load_res6<R>(rel, (size_t)a.idx[c + q], v[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (c + q < end) {
-#pragma unroll
-            for (int f = 0; f < 6; ++f) r[f] += (double)v[q][f];
-          }
-      }
-    } else {
-      // FP64 residual rows: full groups of 4, then one at a time (a predicated group's 24
-      // doubles do not fit the register budget)
-      for (; c + 4 <= end; c += 4) {
-        R v[4][6];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) load_res6<R>(rel, (size_t)a.idx[c + q], v[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int f = 0; f < 6; ++f) r[f] += (double)v[q][f];
-      }
-      for (; c < end; ++c) {
-        R v[6];
-        load_res6<R>(rel, (size_t)a.idx[c], v);
-#pragma unroll
-        for (int f = 0; f < 6; ++f) r[f] += (double)v[f];
-      }
-    }
+    gather_rows<R>(rel, a.idx, beg, end, r);
     if (a.src) {
       // mom_source_const_vect (elem_source.f90:20-55): - sum_e gpvol s = - Ml s on the momentum
 #pragma unroll
-      for (int d = 0; d < 3; ++d) r[1 + d] -= ml * a.src[d * N + n];
+      for (int d = 0; d < 3; ++d) r[1 + d] -= a.Ml[n] * a.src[d * N + n];
     }
     if (a.wm) {
       // wall model: the modelled shear added to Rdiff_mom (time_integ.f90:334-357)
@@ -144,7 +110,7 @@ __device__ __forceinline__ bool gather_rk_node(const GatherArgs& a, int n, doubl
       for (int d = 0; d < 3; ++d) r[1 + d] += a.wm[d * N + n];
     }
 #pragma unroll
-    for (int f = 0; f < 6; ++f) r[f] = r[f] / ml;
+    for (int f = 0; f < 6; ++f) r[f] *= iml;
     if constexpr (STAGE == 0) {
 #pragma unroll
       for (int f = 0; f < 6; ++f)
@@ -181,8 +147,8 @@ __device__ __forceinline__ bool gather_rk_node(const GatherArgs& a, int n, doubl
         const double pr = rho * (g - 1.0) * ei;
         const double cs = sqrt(g * pr * irho);
         umag = sqrt(umag);
-        const double T = pr * irho / a.Rgas;
-        const double eta = (rho / (g - 1.0)) * (log(pr) - g * log(rho));
+        const double T = pr * irho * a.inv_Rgas;
+        const double eta = rho * a.inv_gm1 * (log(pr) - g * log(rho));
         a.u0[n] = u0; a.u1[n] = u1; a.u2[n] = u2;
         a.e_int[n] = ei; a.pr[n] = pr; a.csound[n] = cs; a.machno[n] = umag / cs;
         a.Tem[n] = T; a.eta[n] = eta;
