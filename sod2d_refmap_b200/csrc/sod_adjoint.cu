@@ -394,8 +394,10 @@ __global__ void k_seed(int64_t N, Cols5 src, const double* __restrict__ Ml, cons
 }
 
 // Ordered gather of the element-node adjoints [e][6][64] (ascending element order, like the
-// forward assembly), plus extra ([5][npoin], or null); Ybar = sum; out = Ybar (mode 0) or
-// acc += Ybar (mode 1, acc = out); when wnext is set: wnext = -dt (cb * ybar + ca * Ybar) / Ml.
+// forward assembly), plus extra ([5][npoin], or null); Ybar = sum; out = Ybar (mode 0),
+// out += Ybar (mode 1) or out = ybar + Ybar (mode 2: the first accumulation, so that out needs no copy
+// of ybar before it and may be the array ybar was kept from); when wnext is set:
+// wnext = -dt (cb * ybar + ca * Ybar) / Ml.
 __global__ void __launch_bounds__(256) k_gather_vjp(int64_t N, const int32_t* __restrict__ ptr,
                                                     const int32_t* __restrict__ idx, const double* __restrict__ el,
                                                     MCols5 out, int mode, const double* __restrict__ ybar,
@@ -404,27 +406,26 @@ __global__ void __launch_bounds__(256) k_gather_vjp(int64_t N, const int32_t* __
                                                     const double* __restrict__ extra) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  double r[5] = {0, 0, 0, 0, 0};
-  const int beg = ptr[n], end = ptr[n + 1];
-  for (int c = beg; c < end; ++c) {
-    double v[6];
-    load_res6<double>(el, (size_t)idx[c], v);
-#pragma unroll
-    for (int f = 0; f < 5; ++f) r[f] += v[f];
-  }
+  double r[6] = {0, 0, 0, 0, 0, 0};
+  gather_rows<double>(el, idx, ptr[n], ptr[n + 1], r);
   if (extra) {  // the wall model's node-level adjoint
 #pragma unroll
     for (int f = 0; f < 5; ++f) r[f] += extra[f * N + n];
   }
+  double yb[5];
+  if (wnext || mode == 2) {
+#pragma unroll
+    for (int f = 0; f < 5; ++f) yb[f] = ybar[f * N + n];
+  }
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
-    if (mode == 1) out.c[f][n] += r[f];
-    else out.c[f][n] = r[f];
+    if (mode == 0) out.c[f][n] = r[f];
+    else out.c[f][n] = (mode == 1 ? out.c[f][n] : yb[f]) + r[f];
   }
   if (wnext) {
     const double sc = -(*dt) / Ml[n];
 #pragma unroll
-    for (int f = 0; f < 5; ++f) wnext[f * N + n] = sc * (cb * ybar[f * N + n] + ca * r[f]);
+    for (int f = 0; f < 5; ++f) wnext[f * N + n] = sc * (cb * yb[f] + ca * r[f]);
   }
 }
 
@@ -457,14 +458,8 @@ __global__ void __launch_bounds__(256) k_stage_state(int64_t N, const int32_t* _
                                                      const double* __restrict__ wmc, double* __restrict__ ys) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  double r[5] = {0, 0, 0, 0, 0};
-  const int beg = ptr[n], end = ptr[n + 1];
-  for (int c = beg; c < end; ++c) {
-    double v[6];
-    load_res6<double>(el, (size_t)idx[c], v);
-#pragma unroll
-    for (int f = 0; f < 5; ++f) r[f] += v[f];
-  }
+  double r[6] = {0, 0, 0, 0, 0, 0};
+  gather_rows<double>(el, idx, ptr[n], ptr[n + 1], r);
   // same operation order as the forward stage gather, so the stage states match it bit for bit
   const double ml = Ml[n];
   if (src) {
@@ -492,14 +487,8 @@ __global__ void __launch_bounds__(256) k_final_pre(int64_t N, const int32_t* __r
                                                    double* __restrict__ zf) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  double r[5] = {0, 0, 0, 0, 0};
-  const int beg = ptr[n], end = ptr[n + 1];
-  for (int c = beg; c < end; ++c) {
-    double v[6];
-    load_res6<double>(el, (size_t)idx[c], v);
-#pragma unroll
-    for (int f = 0; f < 5; ++f) r[f] += v[f];
-  }
+  double r[6] = {0, 0, 0, 0, 0, 0};
+  gather_rows<double>(el, idx, ptr[n], ptr[n + 1], r);
   const double ml = Ml[n];
   if (src) {
 #pragma unroll
@@ -769,9 +758,11 @@ int sod_rk4_step_vjp(SodMesh* m, const double* rho, const double* q, const doubl
   SOD_CHECK_LAUNCH();
   keep = MCols5{{yb, yb + N, yb + 2 * N, yb + 3 * N, yb + 4 * N}};
   MCols5 acc{{out_rho, out_q, out_q + N, out_q + 2 * N, out_E}};
-  // acc = ybar (copied from the kept columns, so out may alias bar)
-  for (int f = 0; f < 5; ++f)
-    SOD_CUDA(cudaMemcpyAsync(acc.c[f], keep.c[f], N * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  // with boundaries acc = ybar (copied from the kept columns, so out may alias bar); without, the
+  // first stage's gather writes ybar + Ybar4
+  if (bc)
+    for (int f = 0; f < 5; ++f)
+      SOD_CUDA(cudaMemcpyAsync(acc.c[f], keep.c[f], N * sizeof(double), cudaMemcpyDeviceToDevice, st));
   if (slip) {
     // the update's slip walls read the velocity q/rho of y0 itself
     rc = bc_slip_push(m, rho, q, out_rho, out_q, st);
@@ -793,7 +784,7 @@ int sod_rk4_step_vjp(SodMesh* m, const double* rho, const double* q, const doubl
     }
     const int t = 4 - stage;
     if (!bc) {
-      k_gather_vjp<<<nblk(N), 256, 0, st>>>(N, m->n2e_ptr, m->n2e, rel, acc, 1, yb, m->Ml, dt_dev, cb[t], ca[t],
+      k_gather_vjp<<<nblk(N), 256, 0, st>>>(N, m->n2e_ptr, m->n2e, rel, acc, t == 0 ? 2 : 1, yb, m->Ml, dt_dev, cb[t], ca[t],
                                              stage > 1 ? w : nullptr, wmb);
       SOD_CHECK_LAUNCH();
     } else {
