@@ -2,7 +2,14 @@
 // reference's inputs independent (e.g. full_convec_ijk takes u and q separately, and the
 // energy-like field E as given) and writes fully overwritten nodal outputs.  Element work
 // runs one CTA per element (64 threads = gauss points) in FP64, assembly is the same ordered
-// CSR gather as the fused path.
+// CSR gather of node-major residual rows as the fused path.
+//
+// The element kernels make one pass over the 12 line points of each node: the products of a
+// quartet share the line point's contravariant velocities V(m) = sum_c He(c,dir)(x) u_c(m) and
+// W(m) (of q), formed with the output point's metric, so nothing but the nodal fields is staged and
+// no product is differentiated by itself.  Lanes are ordered (i0 j0 i1 j1 k): a warp's xi and eta line
+// loads then cost one shared-memory wavefront each (see sod_rhs.cu).  20^3 elements:
+// convection 78 -> 25 us, diffusion 35 -> 27, scalar 22 -> 17, gather of 5 fields 15 -> 9.
 #include "sod_internal.cuh"
 #include <cmath>
 
@@ -10,23 +17,22 @@ namespace sod {
 
 int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st);
 
-__device__ __forceinline__ void giso_d(const double* f, int i, int j, int k, const double (&D)[NP1][NP1],
-                                       double& gx, double& gy, double& gz) {
-  gx = gy = gz = 0.0;
-#pragma unroll
-  for (int m = 0; m < NP1; ++m) {
-    gx += D[i][m] * f[sidx(m, j, k)];
-    gy += D[j][m] * f[sidx(i, m, k)];
-    gz += D[k][m] * f[sidx(i, j, m)];
-  }
-}
-__device__ __forceinline__ double divT_d(const double* fx, const double* fy, const double* fz, int i, int j, int k,
-                                         const double (&D)[NP1][NP1]) {
-  double s = 0.0;
-#pragma unroll
-  for (int m = 0; m < NP1; ++m)
-    s += D[m][i] * fx[sidx(m, j, k)] + D[m][j] * fy[sidx(i, m, k)] + D[m][k] * fz[sidx(i, j, m)];
-  return s;
+// the thread's point in the lane order (i0 j0 i1 j1 k), and its three lines in a staged field
+struct Point {
+  int i, j, k, d, s;
+  int row[3], line[3];
+};
+__host__ __device__ constexpr int line_stride(int dir) { return dir == 0 ? 1 : (dir == 1 ? 4 : PLANE); }
+__device__ __forceinline__ Point point_of(int lt) {
+  Point p;
+  p.i = (lt & 1) | ((lt >> 1) & 2);
+  p.j = ((lt >> 1) & 1) | ((lt >> 2) & 2);
+  p.k = lt >> 4;
+  p.d = p.i + 4 * p.j + 16 * p.k;
+  p.s = sidx(p.i, p.j, p.k);
+  p.row[0] = p.i; p.row[1] = p.j; p.row[2] = p.k;
+  p.line[0] = sidx(0, p.j, p.k); p.line[1] = sidx(p.i, 0, p.k); p.line[2] = sidx(p.i, p.j, 0);
+  return p;
 }
 
 struct RefArgs {
@@ -39,189 +45,250 @@ struct RefArgs {
   const double *rho_n, *Tem, *mu_fluid;         // diffusion
   const double *mue, *musgs;                    // internal layout [e][64]
   double Cp, Pr, c_rho, c_ener;
-  double* rel;                                  // [e][6][64]
+  double* rel;                                  // rows [(e*64 + d)*6 + f]
 };
 
 // full_convec_ijk (elem_convec.f90:241-435); TOTH: full_convec_ijk_H (elem_convec.f90:48-187),
 // whose energy residual is 0.5 (div((E + p) u) + (E + p) div u + u . grad(E + p)) with E the
-// total energy; mass and momentum are the same in both
+// total energy; mass and momentum are the same in both.  Both energy quartets (E and k = |u|^2/2, the
+// same form) are taken at once on H = E + k.
 template <bool TOTH>
-__global__ void __launch_bounds__(64) k_convec_ref(const RefArgs a) {
-  __shared__ double f[42][FSTRIDE];
-  __shared__ DMat Ds;
-  const int e = blockIdx.x, d = threadIdx.x;
-  const int i = d & 3, j = (d >> 2) & 3, k = d >> 4, s = sidx(i, j, k);
-  if (d < 16) Ds.d[d >> 2][d & 3] = a.D.d[d >> 2][d & 3];
-  const int n = a.econn[(int64_t)e * NN + d];
+__global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefArgs a) {
+  __shared__ double f[9][FSTRIDE];  // rho, p, H (TOTH: p + E), u, q
+  __shared__ double Ds[16];
+  const int e = blockIdx.x;
+  const Point p = point_of(threadIdx.x);
+  if (threadIdx.x < 16) Ds[threadIdx.x] = a.D.d[threadIdx.x >> 2][threadIdx.x & 3];
+  const int n = a.econn[(int64_t)e * NN + p.d];
   const int64_t N = a.npoin;
-  double u[3], q[3];
-  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; q[c] = a.q[n + N * c]; }
-  const double rho = a.rho[n], El = a.E[n], pr = a.pr[n];
-  double kl = 0.0;
-  for (int c = 0; c < 3; ++c) kl = kl + u[c] * u[c] * 0.5;
-  // fields: 0 rho,1 p,2 E,3 rhoE,4 k,5 rhok, 6-8 u, 9-11 q, 12-14 fe, 15-17 fue, 18-20 fk, 21-23 fuk,
-  //         24-32 F=q x u, 33-41 Fuu = u x u
-  // TOTH: field 2 holds p + E and fields 12-14 (E + p) u
-  f[0][s] = rho; f[1][s] = pr; f[2][s] = TOTH ? pr + El : El; f[3][s] = rho * El; f[4][s] = kl; f[5][s] = rho * kl;
-  for (int c = 0; c < 3; ++c) {
-    f[6 + c][s] = u[c]; f[9 + c][s] = q[c];
-    f[12 + c][s] = TOTH ? (El + pr) * u[c] : rho * El * u[c]; f[15 + c][s] = El * u[c];
-    f[18 + c][s] = rho * kl * u[c]; f[21 + c][s] = kl * u[c];
-    for (int c2 = 0; c2 < 3; ++c2) { f[24 + 3 * c + c2][s] = q[c] * u[c2]; f[33 + 3 * c + c2][s] = u[c] * u[c2]; }
-  }
-  __syncthreads();
   const double* G = a.geo + (int64_t)e * NGEO * NN;
   double H[9];
-  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + d];
-  const double gpv = G[9 * NN + d];
-  auto grad = [&](int fi, double* o) {
-    double gx, gy, gz;
-    giso_d(f[fi], i, j, k, Ds.d, gx, gy, gz);
-    for (int r = 0; r < 3; ++r) o[r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
-  };
-  double gRho[3], gP[3], gE[3], gRE[3], gk[3], gRk[3], gU[3][3], gQ[3][3];
-  grad(0, gRho); grad(1, gP); grad(2, gE); grad(3, gRE); grad(4, gk); grad(5, gRk);
-  for (int c = 0; c < 3; ++c) { grad(6 + c, gU[c]); grad(9 + c, gQ[c]); }
-  auto divg = [&](int fi) {
-    double sdiv = 0.0;
-    for (int c = 0; c < 3; ++c) { double g3[3]; grad(fi + c, g3); sdiv += g3[c]; }
-    return sdiv;
-  };
-  const double divFe = divg(12), divFue = divg(15), divFk = divg(18), divFuk = divg(21);
-  double divF[3], divFuu[3];
-  for (int c = 0; c < 3; ++c) { divF[c] = divg(24 + 3 * c); divFuu[c] = divg(33 + 3 * c); }
-  const double divU = gU[0][0] + gU[1][1] + gU[2][2];
-  const double divQ = gQ[0][0] + gQ[1][1] + gQ[2][2];
-  double Rm = 0.5 * (divQ + rho * divU);
-  double Re = TOTH ? 0.5 * (divFe + (El + pr) * divU)
-                   : 0.25 * (divFe + El * divQ + rho * El * divU + rho * divFue) +
-                         0.25 * (divFk + kl * divQ + rho * kl * divU + rho * divFuk);
-  double Rmo[3];
-  for (int c = 0; c < 3; ++c) {
-    Rmo[c] = 0.25 * (divF[c] + u[c] * divQ + q[c] * divU + rho * divFuu[c]) + gP[c];
-    Rm = Rm + 0.5 * (u[c] * gRho[c]);
-    if (TOTH)
-      Re = Re + 0.5 * (u[c] * gE[c]);
-    else
-      Re = Re + 0.25 * (q[c] * gE[c] + u[c] * gRE[c] + El * u[c] * gRho[c]) +
-           0.25 * (q[c] * gk[c] + u[c] * gRk[c] + kl * u[c] * gRho[c]);
-    for (int c2 = 0; c2 < 3; ++c2) Rmo[c] = Rmo[c] + 0.25 * (u[c] * u[c2] * gRho[c2] + q[c2] * gU[c][c2] + u[c2] * gQ[c][c2]);
+#pragma unroll
+  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + p.d];
+  const double gpv = G[9 * NN + p.d];
+  double u[3], q[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; q[c] = a.q[n + N * c]; }
+  const double rho = a.rho[n], El = a.E[n], pr = a.pr[n];
+  const double Hx = TOTH ? pr + El : El + 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  f[0][p.s] = rho; f[1][p.s] = pr; f[2][p.s] = Hx;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { f[3 + c][p.s] = u[c]; f[6 + c][p.s] = q[c]; }
+  __syncthreads();
+  double divU = 0.0, divQ = 0.0, ugr = 0.0;      // div u, div q, u.grad rho
+  double A[3] = {0, 0, 0}, B[3] = {0, 0, 0};     // div(q_c u) + rho div(u_c u); q.grad u_c + u.grad q_c
+  double gP[3] = {0, 0, 0};
+  double Ea = 0.0, Er = 0.0, Eb = 0.0;           // div(rho H u) + rho div(H u) (TOTH: div(H u)) less H times (Er = div(rho u), ..); the advective rest
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const double h0 = H[dir], h1 = H[3 + dir], h2 = H[6 + dir];
+    const double Vx = h0 * u[0] + h1 * u[1] + h2 * u[2], Wx = h0 * q[0] + h1 * q[1] + h2 * q[2];
+    double lu[3] = {0, 0, 0}, lq[3] = {0, 0, 0}, lr = 0.0, lp = 0.0, lH = 0.0, lrH = 0.0;
+#pragma unroll
+    for (int m = 0; m < NP1; ++m) {
+      const double* v = &f[0][0] + p.line[dir] + m * line_stride(dir);
+      const double w = Ds[4 * p.row[dir] + m];
+      const double u_[3] = {v[3 * FSTRIDE], v[4 * FSTRIDE], v[5 * FSTRIDE]};
+      const double q_[3] = {v[6 * FSTRIDE], v[7 * FSTRIDE], v[8 * FSTRIDE]};
+      const double r_ = v[0], H_ = v[2 * FSTRIDE];
+      const double wV = w * (h0 * u_[0] + h1 * u_[1] + h2 * u_[2]);
+      lr += w * r_;
+      lp += w * v[FSTRIDE];
+      // H by its difference to the own point: the constant part of div(rho H u) + rho div(H u) and of
+      // u.grad(rho H) is H times small sums, formed once below
+      const double dH = H_ - Hx;
+      lH += w * dH;
+      if (TOTH) {
+        Ea += wV * dH;
+      } else {
+        const double wVr = wV * r_;
+        Er += wVr;
+        Ea += (wVr + wV * rho) * dH;
+        lrH += (w * r_) * dH;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        A[c] += wV * (q_[c] + rho * u_[c]);
+        lu[c] += w * u_[c];
+        lq[c] += w * q_[c];
+      }
+    }
+    divU += h0 * lu[0] + h1 * lu[1] + h2 * lu[2];
+    divQ += h0 * lq[0] + h1 * lq[1] + h2 * lq[2];
+    ugr += Vx * lr;
+    gP[0] += h0 * lp;
+    gP[1] += h1 * lp;
+    gP[2] += h2 * lp;
+    Eb += TOTH ? Vx * lH : Wx * lH + Vx * lrH;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) B[c] += Wx * lu[c] + Vx * lq[c];
   }
-  double* out = a.rel + (int64_t)e * NRES * NN + d;
-  out[0] = gpv * Rm; out[NN] = gpv * Rmo[0]; out[2 * NN] = gpv * Rmo[1]; out[3 * NN] = gpv * Rmo[2];
-  out[4 * NN] = gpv * Re; out[5 * NN] = 0.0;
+  const double Rm = 0.5 * (divQ + rho * divU + ugr);
+  const double Re = TOTH ? 0.5 * (Ea + 2.0 * Hx * divU + Eb)
+                         : 0.25 * (Ea + Eb + Hx * (Er + divQ + 2.0 * (rho * divU + ugr)));
+  double Rmo[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) Rmo[c] = 0.25 * (A[c] + u[c] * divQ + q[c] * divU + B[c] + u[c] * ugr) + gP[c];
+  store_res6<double>(a.rel, (size_t)e * NN + p.d, gpv * Rm, gpv * Rmo[0], gpv * Rmo[1], gpv * Rmo[2], gpv * Re, 0.0);
 }
 
 // generic_scalar_convec_ijk (elem_convec.f90:488-556)
-__global__ void __launch_bounds__(64) k_scalar_ref(const RefArgs a) {
+__global__ void __launch_bounds__(64) k_scalar_ref(const __grid_constant__ RefArgs a) {
   __shared__ double f[7][FSTRIDE];
-  __shared__ DMat Ds;
-  const int e = blockIdx.x, d = threadIdx.x;
-  const int i = d & 3, j = (d >> 2) & 3, k = d >> 4, s = sidx(i, j, k);
-  if (d < 16) Ds.d[d >> 2][d & 3] = a.D.d[d >> 2][d & 3];
-  const int n = a.econn[(int64_t)e * NN + d];
+  __shared__ double Ds[16];
+  const int e = blockIdx.x;
+  const Point p = point_of(threadIdx.x);
+  if (threadIdx.x < 16) Ds[threadIdx.x] = a.D.d[threadIdx.x >> 2][threadIdx.x & 3];
+  const int n = a.econn[(int64_t)e * NN + p.d];
   const int64_t N = a.npoin;
-  double u[3];
-  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; f[1 + c][s] = u[c]; f[4 + c][s] = a.q[n + N * c]; }
-  const double eta = a.E[n];
-  f[0][s] = eta;
-  __syncthreads();
   const double* G = a.geo + (int64_t)e * NGEO * NN;
   double H[9];
-  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + d];
-  double gx, gy, gz, gE[3], divU = 0.0, divFe = 0.0;
-  giso_d(f[0], i, j, k, Ds.d, gx, gy, gz);
-  for (int r = 0; r < 3; ++r) gE[r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
-  for (int c = 0; c < 3; ++c) {
-    giso_d(f[1 + c], i, j, k, Ds.d, gx, gy, gz);
-    divU += H[3 * c] * gx + H[3 * c + 1] * gy + H[3 * c + 2] * gz;
-    giso_d(f[4 + c], i, j, k, Ds.d, gx, gy, gz);
-    divFe += H[3 * c] * gx + H[3 * c + 1] * gy + H[3 * c + 2] * gz;
+#pragma unroll
+  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + p.d];
+  const double gpv = G[9 * NN + p.d];
+  double u[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; f[1 + c][p.s] = u[c]; f[4 + c][p.s] = a.q[n + N * c]; }
+  const double eta = a.E[n];
+  f[0][p.s] = eta;
+  __syncthreads();
+  double div = 0.0, divU = 0.0, adv = 0.0;
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    double le = 0.0, lu[3] = {0, 0, 0}, lq[3] = {0, 0, 0};
+#pragma unroll
+    for (int m = 0; m < NP1; ++m) {
+      const double* v = &f[0][0] + p.line[dir] + m * line_stride(dir);
+      const double w = Ds[4 * p.row[dir] + m];
+      le += w * v[0];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) { lu[c] += w * v[(1 + c) * FSTRIDE]; lq[c] += w * v[(4 + c) * FSTRIDE]; }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      divU += H[3 * c + dir] * lu[c];
+      div += H[3 * c + dir] * lq[c];
+      adv += (H[3 * c + dir] * u[c]) * le;
+    }
   }
-  double Re = 0.5 * (divFe + eta * divU);
-  for (int c = 0; c < 3; ++c) Re = Re + 0.5 * (u[c] * gE[c]);
-  double* out = a.rel + (int64_t)e * NRES * NN + d;
-  for (int fld = 0; fld < 5; ++fld) out[fld * NN] = 0.0;
-  out[5 * NN] = G[9 * NN + d] * Re;
+  a.rel[(size_t)e * NN + p.d] = gpv * (0.5 * (div + eta * divU + adv));  // one value per element node
 }
 
 // full_diffusion_ijk (elem_diffu.f90:44-194)
-__global__ void __launch_bounds__(64) k_diffusion_ref(const RefArgs a) {
-  __shared__ double f[5][FSTRIDE];
+__global__ void __launch_bounds__(64) k_diffusion_ref(const __grid_constant__ RefArgs a) {
+  __shared__ double f[5][FSTRIDE];  // rho, T, u
   __shared__ double V[18][FSTRIDE];
-  __shared__ DMat Ds;
-  const int e = blockIdx.x, d = threadIdx.x;
-  const int i = d & 3, j = (d >> 2) & 3, k = d >> 4, s = sidx(i, j, k);
-  if (d < 16) Ds.d[d >> 2][d & 3] = a.D.d[d >> 2][d & 3];
-  const int n = a.econn[(int64_t)e * NN + d];
+  __shared__ double Ds[16], DTs[16];
+  const int e = blockIdx.x;
+  const Point p = point_of(threadIdx.x);
+  if (threadIdx.x < 16) {
+    Ds[threadIdx.x] = a.D.d[threadIdx.x >> 2][threadIdx.x & 3];
+    DTs[threadIdx.x] = a.D.d[threadIdx.x & 3][threadIdx.x >> 2];
+  }
+  const int n = a.econn[(int64_t)e * NN + p.d];
   const int64_t N = a.npoin;
-  double u[3];
-  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; f[2 + c][s] = u[c]; }
-  f[0][s] = a.rho[n];
-  f[1][s] = a.Tem[n];
-  const double rhon = a.rho_n[n], muf = a.mu_fluid[n];
-  const double mue = a.mue[(int64_t)e * NN + d];
-  const double musgs = a.musgs ? a.musgs[(int64_t)e * NN + d] : 0.0;
-  __syncthreads();
   const double* G = a.geo + (int64_t)e * NGEO * NN;
   double H[9];
-  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + d];
-  const double gpv = G[9 * NN + d];
-  double gx, gy, gz, gRho[3], gT[3], gU[3][3];
-  giso_d(f[0], i, j, k, Ds.d, gx, gy, gz);
-  for (int r = 0; r < 3; ++r) gRho[r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
-  giso_d(f[1], i, j, k, Ds.d, gx, gy, gz);
-  for (int r = 0; r < 3; ++r) gT[r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
-  for (int c = 0; c < 3; ++c) {
-    giso_d(f[2 + c], i, j, k, Ds.d, gx, gy, gz);
-    for (int r = 0; r < 3; ++r) gU[c][r] = H[3 * r] * gx + H[3 * r + 1] * gy + H[3 * r + 2] * gz;
+#pragma unroll
+  for (int c = 0; c < 9; ++c) H[c] = G[c * NN + p.d];
+  const double gpv = G[9 * NN + p.d];
+  double u[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; f[2 + c][p.s] = u[c]; }
+  f[0][p.s] = a.rho[n];
+  f[1][p.s] = a.Tem[n];
+  const double rhon = a.rho_n[n], muf = a.mu_fluid[n];
+  const double mue = a.mue[(int64_t)e * NN + p.d];
+  const double musgs = a.musgs ? a.musgs[(int64_t)e * NN + p.d] : 0.0;
+  __syncthreads();
+  double gRho[3] = {0, 0, 0}, gT[3] = {0, 0, 0}, gU[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    double l[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int m = 0; m < NP1; ++m) {
+      const double* v = &f[0][0] + p.line[dir] + m * line_stride(dir);
+      const double w = Ds[4 * p.row[dir] + m];
+#pragma unroll
+      for (int c = 0; c < 5; ++c) l[c] += w * v[c * FSTRIDE];
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const double h = H[3 * r + dir];
+      gRho[r] += h * l[0];
+      gT[r] += h * l[1];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gU[c][r] += h * l[2 + c];
+    }
   }
   const double divU = gU[0][0] + gU[1][1] + gU[2][2];
-  const double mu_fgp = muf + rhon * musgs, mu_egp = mue;
+  const double mu_fgp = muf + rhon * musgs, mut = mu_fgp + mue;
   const double twoThirds = 2.0 / 3.0;
   double tau[3][3], tauU[3];
+#pragma unroll
   for (int r = 0; r < 3; ++r) {
-    tauU[r] = 0.0;
-    for (int c = 0; c < 3; ++c) {
-      tauU[r] = tauU[r] + (mu_fgp + mu_egp) * (gU[r][c] + gU[c][r]) * u[c];
-      tau[r][c] = (mu_fgp + mu_egp) * (gU[r][c] + gU[c][r]);
-    }
-    tauU[r] = tauU[r] - mu_fgp * twoThirds * divU * u[r];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) tau[r][c] = mut * (gU[r][c] + gU[c][r]);
     tau[r][r] = tau[r][r] - mu_fgp * twoThirds * divU;
+    tauU[r] = tau[r][0] * u[0] + tau[r][1] * u[1] + tau[r][2] * u[2];
   }
-  const double* Vs[6] = {gRho, tauU, gT, tau[0], tau[1], tau[2]};
-  for (int v = 0; v < 6; ++v)
-    for (int dir = 0; dir < 3; ++dir)
-      V[3 * v + dir][s] = gpv * (H[dir] * Vs[v][0] + H[3 + dir] * Vs[v][1] + H[6 + dir] * Vs[v][2]);
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const double h0 = gpv * H[dir], h1 = gpv * H[3 + dir], h2 = gpv * H[6 + dir];
+    auto emit = [&](int v, const double* x) { V[3 * v + dir][p.s] = h0 * x[0] + h1 * x[1] + h2 * x[2]; };
+    emit(0, gRho);
+    emit(1, tauU);
+    emit(2, gT);
+    emit(3, tau[0]);
+    emit(4, tau[1]);
+    emit(5, tau[2]);
+  }
   __syncthreads();
-  double dv[6];
-  for (int v = 0; v < 6; ++v) dv[v] = divT_d(V[3 * v], V[3 * v + 1], V[3 * v + 2], i, j, k, Ds.d);
+  double dv[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir)
+#pragma unroll
+    for (int m = 0; m < NP1; ++m) {
+      const double w = DTs[4 * p.row[dir] + m];
+#pragma unroll
+      for (int v = 0; v < 6; ++v) dv[v] += w * V[3 * v + dir][p.line[dir] + m * line_stride(dir)];
+    }
   const double nu_e = a.c_rho * mue / rhon;
   const double kappa_e = muf * a.Cp / a.Pr + a.c_ener * mue * a.Cp / a.Pr + a.Cp * rhon * musgs / 0.9;
-  double* out = a.rel + (int64_t)e * NRES * NN + d;
-  out[0] = nu_e * dv[0];
-  out[NN] = dv[3]; out[2 * NN] = dv[4]; out[3 * NN] = dv[5];
-  out[4 * NN] = dv[1] + kappa_e * dv[2];
-  out[5 * NN] = 0.0;
+  store_res6<double>(a.rel, (size_t)e * NN + p.d, nu_e * dv[0], dv[3], dv[4], dv[5], dv[1] + kappa_e * dv[2], 0.0);
 }
 
-// ordered gather of selected residual fields, optional /Ml
-__global__ void k_gather_plain(int npoin, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                               const double* __restrict__ rel, const double* __restrict__ Ml, int f0, int nf,
-                               double* o0, double* o1, double* o2, double* o3, double* o4) {
+// ordered gather of the residual rows' five fields
+__global__ void __launch_bounds__(256) k_gather_rows5(int npoin, const int32_t* __restrict__ ptr,
+                                                      const int32_t* __restrict__ idx, const double* __restrict__ rel,
+                                                      double* __restrict__ o0, double* __restrict__ o1,
+                                                      double* __restrict__ o4) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= npoin) return;
-  double r[5] = {0, 0, 0, 0, 0};
-  for (int c = ptr[n]; c < ptr[n + 1]; ++c) {
-    const int pk = idx[c];
-    const double* src = rel + (int64_t)(pk >> 6) * NRES * NN + (pk & 63);
-    for (int f = 0; f < nf; ++f) r[f] += src[(f0 + f) * NN];
+  double r[6] = {0, 0, 0, 0, 0, 0};
+  gather_rows<double>(rel, idx, ptr[n], ptr[n + 1], r);
+  o0[n] = r[0];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o1[n + (int64_t)npoin * c] = r[1 + c];
+  o4[n] = r[4];
+}
+// the same of one value per element node
+__global__ void __launch_bounds__(256) k_gather_one(int npoin, const int32_t* __restrict__ ptr,
+                                                    const int32_t* __restrict__ idx, const double* __restrict__ rel,
+                                                    double* __restrict__ out) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= npoin) return;
+  double s = 0.0;
+  for (int c = ptr[n]; c < ptr[n + 1]; c += 4) {
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c + q < ptr[n + 1]) v[q] = rel[idx[c + q]];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c + q < ptr[n + 1]) s += v[q];
   }
-  double* outs[5] = {o0, o1, o2, o3, o4};
-  for (int f = 0; f < nf; ++f) {
-    double v = Ml ? r[f] / Ml[n] : r[f];
-    if (outs[f]) outs[f][n] = v;
-  }
+  out[n] = s;
 }
 
 // lumped_solver_scal/vect over the working nodes (mod_solver.f90:23-58): rows without elements
@@ -316,10 +383,9 @@ __global__ void k_csr_spmv_legacy(int npoin, const int32_t* __restrict__ rdom, c
   u[r] = s;
 }
 
-static int gather_out(SodMesh* m, const double* Ml, int f0, int nf, double* o0, double* o1, double* o2, double* o3,
-                      double* o4, cudaStream_t st) {
-  k_gather_plain<<<(m->npoin + 255) / 256, 256, 0, st>>>(m->npoin, m->n2e_ptr, m->n2e, (const double*)m->buf.rel, Ml,
-                                                          f0, nf, o0, o1, o2, o3, o4);
+static int gather_out(SodMesh* m, double* Rmass, double* Rmom, double* Rener, cudaStream_t st) {
+  k_gather_rows5<<<(m->npoin + 255) / 256, 256, 0, st>>>(m->npoin, m->n2e_ptr, m->n2e, (const double*)m->buf.rel, Rmass,
+                                                          Rmom, Rener);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
@@ -353,8 +419,7 @@ int sod_full_convec_ijk(SodMesh* m, const double* u, const double* q, const doub
   a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E;
   k_convec_ref<false><<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
-  const size_t N = m->npoin;
-  return gather_out(m, nullptr, 0, 5, Rmass, Rmom, Rmom + N, Rmom + 2 * N, Rener, st);
+  return gather_out(m, Rmass, Rmom, Rener, st);
 }
 
 int sod_full_convec_ijk_H(SodMesh* m, const double* u, const double* q, const double* rho, const double* pr,
@@ -367,8 +432,7 @@ int sod_full_convec_ijk_H(SodMesh* m, const double* u, const double* q, const do
   a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E;
   k_convec_ref<true><<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
-  const size_t N = m->npoin;
-  return gather_out(m, nullptr, 0, 5, Rmass, Rmom, Rmom + N, Rmom + 2 * N, Rener, st);
+  return gather_out(m, Rmass, Rmom, Rener, st);
 }
 
 int sod_generic_scalar_convec_ijk(SodMesh* m, const double* q, const double* eta, const double* u,
@@ -381,7 +445,9 @@ int sod_generic_scalar_convec_ijk(SodMesh* m, const double* q, const double* eta
   a.u = u; a.q = q; a.E = eta;
   k_scalar_ref<<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
-  return gather_out(m, nullptr, 5, 1, Rconvec, nullptr, nullptr, nullptr, nullptr, st);
+  k_gather_one<<<(m->npoin + 255) / 256, 256, 0, st>>>(m->npoin, m->n2e_ptr, m->n2e, (const double*)m->buf.rel, Rconvec);
+  SOD_CHECK_LAUNCH();
+  return SOD_OK;
 }
 
 int sod_full_diffusion_ijk(SodMesh* m, double Cp, double Pr, const double* rho_n, const double* rho,
@@ -406,8 +472,7 @@ int sod_full_diffusion_ijk(SodMesh* m, double Cp, double Pr, const double* rho_n
   k_diffusion_ref<<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
   if (musgs_int) SOD_CUDA(cudaFreeAsync(musgs_int, st));
-  const size_t N = m->npoin;
-  return gather_out(m, nullptr, 0, 5, Rmass, Rmom, Rmom + N, Rmom + 2 * N, Rener, st);
+  return gather_out(m, Rmass, Rmom, Rener, st);
 }
 
 int sod_lumped_solver(SodMesh* m, double* R, int ncomp, sod_stream_t stream) {
