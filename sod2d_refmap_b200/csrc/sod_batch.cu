@@ -16,7 +16,7 @@
 namespace sod {
 int run_step(SodMesh* m, SodState* s, const double* dt_dev, double* dt_next, bool mixed, cudaStream_t st,
              cudaEvent_t* ev, double* stage_store, cudaEvent_t state_done);
-int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st);
+int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st, bool bits_set);
 }  // namespace sod
 
 struct SodBatch {
@@ -328,7 +328,7 @@ int sod_batch_adapt_dt(SodBatch* B, sod_stream_t stream) {
   s.Reta = m->buf.rsum;  // zero residual: only the dt part matters here
   SOD_CUDA(cudaMemsetAsync(s.Reta, 0, sizeof(double) * m->npoin, st));
   SOD_CUDA(cudaMemsetAsync(m->member_scal, 0, sizeof(double) * 2 * m->nmember, st));
-  rc = launch_visc_dt(m, &s, B->dt, nullptr, st);
+  rc = launch_visc_dt(m, &s, B->dt, nullptr, st, false);
   m->mue_int = save;
   return rc;
 }

@@ -278,6 +278,10 @@ __global__ void __launch_bounds__(64 * EPB) k_stage_fused(const StageArgs p) {
 template <typename R, int STAGE>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? SOD_KG_MIN_BLOCKS : SOD_KG_MIN_BLOCKS_F64) k_gather_rk(const GatherArgs a) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (STAGE == 4) {
+    // the entropy viscosity that follows reduces the next time step into these (1.4e306 each)
+    if (n < a.ndt) a.dt_bits[n] = __longlong_as_double(0x7f7f7f7f7f7f7f7fll);
+  }
   double eta_n = 0.0;
   const bool act = gather_rk_node<R, STAGE>(a, n, eta_n);
   if constexpr (STAGE == 4) {
@@ -484,15 +488,54 @@ static void fill_gather_args(SodMesh* m, int stage, GatherArgs& a) {
   a.scal = m->buf.scal;
   a.src = m->nmember > 0 ? nullptr : m->source;
   a.wm = (m->nmember > 0 || m->wmodel.nw == 0) ? nullptr : m->wmodel.contrib;
+  a.dt_bits = m->nmember > 0 ? m->member_dt_bits : m->buf.scal + 3;
+  a.ndt = m->nmember > 0 ? m->nmember : 1;
   if (stage >= 1) {
     a.b_cur = kB[stage - 1];
     a.a_next = stage < 4 ? kA[stage] : 0.0;
   }
 }
 
+// The entropy normalisation from the stage-4 gather's block sums, in a fixed order.
+__global__ void __launch_bounds__(1024) k_eta_combine(int nblk, int nwork, int normalise, const double* __restrict__ red,
+                                                      double* __restrict__ scal) {
+  __shared__ double sh[3 * 32];
+  double s = 0.0, mx = -1e300, mn = 1e300;
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    s += red[3 * b];
+    mx = fmax(mx, red[3 * b + 1]);
+    mn = fmin(mn, red[3 * b + 2]);
+  }
+  block_reduce3(s, mx, mn, sh);
+  if (threadIdx.x == 0) {
+    if (normalise) {
+      const double mean = s / (double)nwork;
+      scal[0] = mean;
+      scal[1] = fmax(mx - mean, mean - mn);
+    } else {
+      scal[0] = 0.0;
+      scal[1] = 1.0;
+    }
+  }
+}
+
+// Stage 4 forms the entropy normalisation too.  While its blocks are all resident at once (one wave,
+// kOneWave), the last of them does it; beyond, every block would hold its SM slot for the fence and the
+// atomic (~1 us of a ~4 us block), so the block sums go to a launch of their own: 64^3, 27,648 blocks,
+// 458 -> 368 us mixed for 17 us more.
+constexpr int kOneWave = 148 * 4;
 int launch_gather(SodMesh* m, bool mixed, int stage, GatherArgs& a, cudaStream_t st) {
   fill_gather_args(m, stage, a);
-  return mixed ? launch_gather_t<float>(stage, a, st) : launch_gather_t<double>(stage, a, st);
+  const int nblk = (a.npoin + 255) / 256;
+  const bool apart = stage == 4 && !a.member_reduce && nblk > kOneWave;
+  if (apart) a.counter = nullptr;
+  if (int rc = mixed ? launch_gather_t<float>(stage, a, st) : launch_gather_t<double>(stage, a, st)) return rc;
+  if (apart) {
+    k_eta_combine<<<1, 1024, 0, st>>>(nblk, a.nwork, a.normalise, a.red, a.scal);
+    SOD_CHECK_LAUNCH();
+  }
+  return SOD_OK;
 }
 
 // LES is on for a step when the parameters ask for it and the state carries mu_sgs
@@ -539,10 +582,11 @@ static ViscArgs make_visc_args(SodMesh* m, const SodState* s, double* dt_out, fl
   return v;
 }
 
-int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st) {
+// bits_set: the stage-4 gather before it has preset dt_bits
+int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st, bool bits_set) {
   const ViscArgs v = make_visc_args(m, s, dt_out, mue32);
   const int nm = m->nmember > 0 ? m->nmember : 1;
-  if (dt_out) SOD_CUDA(cudaMemsetAsync(v.dt_bits, 0x7F, sizeof(double) * nm, st));  // 1.38e306 each
+  if (dt_out && !bits_set) SOD_CUDA(cudaMemsetAsync(v.dt_bits, 0x7F, sizeof(double) * nm, st));  // 1.38e306 each
   const int grid = (m->nelem + KV_WARPS - 1) / KV_WARPS;
   k_visc_dt<<<grid, 32 * KV_WARPS, 0, st>>>(v);
   SOD_CHECK_LAUNCH();
@@ -741,7 +785,7 @@ int run_step(SodMesh* m, SodState* s, const double* dt_dev, double* dt_next, boo
     rc = launch_sgs(m, s->u, st);
     if (rc) return rc;
   }
-  rc = launch_visc_dt(m, &loc, dt_next, mixed ? m->mue32 : nullptr, st);
+  rc = launch_visc_dt(m, &loc, dt_next, mixed ? m->mue32 : nullptr, st, true);
   if (ev) cudaEventRecord(ev[17], st);
   return rc;
 }

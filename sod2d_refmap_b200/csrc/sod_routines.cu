@@ -15,7 +15,7 @@
 
 namespace sod {
 
-int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st);
+int launch_visc_dt(SodMesh* m, const SodState* s, double* dt_out, float* mue32, cudaStream_t st, bool bits_set);
 
 // the thread's point in the lane order (i0 j0 i1 j1 k), and its three lines in a staged field
 struct Point {
@@ -506,7 +506,7 @@ int sod_smart_visc_spectral(SodMesh* m, const double* Reta, const double* rho, c
   s.csound = const_cast<double*>(csound);
   s.Tem = const_cast<double*>(Tem);
   s.mu_fluid = const_cast<double*>(rho);  // unused without dt
-  rc = launch_visc_dt(m, &s, nullptr, nullptr, st);
+  rc = launch_visc_dt(m, &s, nullptr, nullptr, st, false);
   if (rc) return rc;
   return mesh_internal_to_ref_elem(m, m->mue_int, mu_e, st);
 }

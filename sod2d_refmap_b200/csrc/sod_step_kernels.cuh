@@ -36,10 +36,12 @@ struct GatherArgs {
   const double* mu_factor;
   double gamma, inv_Rgas, inv_gm1;  // 1/Rgas, 1/(gamma-1)
   double* red;              // partials [3*nblocks]
-  unsigned int* counter;
+  unsigned int* counter;    // stage 4: blocks done, or null (k_eta_combine reduces)
   unsigned int* nonfinite;  // raised by stage 4 on a NaN/Inf in the new rho, q, E
   double* scal;             // [0] eta mean, [1] eta norm
   int normalise;
+  double* dt_bits;          // stage 4: preset for the time-step reduction that follows it
+  int ndt;                  // its length (1, or the ensemble's members; 0: not preset)
   const double* src;        // momentum source term (npoin,3) or null
   const double* wm;         // wall-model momentum terms (npoin,3) or null
 };
@@ -162,9 +164,9 @@ __device__ __forceinline__ bool gather_rk_node(const GatherArgs& a, int n, doubl
 }
 
 // The STAGE 4 entropy normalisation (mod_entropy_viscosity.f90:43-66) over the grid: block sums
-// of (eta, max, min) into red[blockIdx.x], then the last block to finish reduces them in a fixed
-// order into scal[0] (mean) and scal[1] (max deviation).  Every thread of the block calls it.
-// sh: 3 doubles per warp.
+// of (eta, max, min) into red[blockIdx.x], then the last block to finish (none without a counter:
+// k_eta_combine follows) reduces them in a fixed order into scal[0] (mean) and scal[1] (max
+// deviation).  Every thread of the block calls it.  sh: 3 doubles per warp.
 __device__ __forceinline__ void gather_eta_reduce(const GatherArgs& a, double s, double mx, double mn, double* sh) {
   __shared__ bool last;
   // entropy normalisation (mod_entropy_viscosity.f90:43-66): sum, max, min of eta
@@ -173,9 +175,12 @@ __device__ __forceinline__ void gather_eta_reduce(const GatherArgs& a, double s,
     a.red[3 * blockIdx.x] = s;
     a.red[3 * blockIdx.x + 1] = mx;
     a.red[3 * blockIdx.x + 2] = mn;
-    __threadfence();
-    unsigned int done = atomicAdd(a.counter, 1u);
-    last = (done == gridDim.x - 1);
+    last = false;
+    if (a.counter) {
+      __threadfence();
+      unsigned int done = atomicAdd(a.counter, 1u);
+      last = (done == gridDim.x - 1);
+    }
   }
   __syncthreads();
   if (last) {
