@@ -41,13 +41,13 @@ constexpr int kBlock = 256;
 constexpr int EPB = 4;      // elements per CTA of the element kernels
 constexpr int NSTAGE = 4;   // cp.async ring stages of the streamed element kernel
 constexpr int kRingCtas = 3; // its resident CTAs per SM (3 x 64.6 KB shared memory in FP64)
-constexpr int kGather = 8;   // residual loads in flight per node in the gather
+constexpr int kGather = 4;   // residual loads in flight per node in the gather (two nodes at a time)
 constexpr int NMET = 6;     // M00, M01, M02, M11, M12, M22
 constexpr int kBatch = 16;  // CG iterations per graph replay
 
 // device scalar slots
 enum {
-  S_Q1 = 0, S_Q2, S_T1, S_NUM, S_ALPHA, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_COUNT
+  S_Q1 = 0, S_Q2, S_T1, S_NUM, S_ALPHA, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD, S_COUNT
 };
 
 template <typename T>
@@ -64,15 +64,14 @@ struct SodPoisson {
   int pin = 0;
   double* met = nullptr;   // [e][6][64]  gpvol He^T He
   float* met32 = nullptr;
-  double* diag = nullptr;
-  float* diag32 = nullptr;
+  double *diag = nullptr, *idiag = nullptr;   // Jacobi diagonal M and 1 / M
+  float* idiag32 = nullptr;
   void* rel = nullptr;     // element residuals [e*64 + d] (double, or float for the FP32 sweeps)
   // CG work vectors (FP64) and inner FP32 vectors
-  double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *b = nullptr;
-  float *r32 = nullptr, *p32 = nullptr, *q32 = nullptr, *z32 = nullptr, *e32 = nullptr;
-  double* part = nullptr;  // block partials [3][nblk]
-  unsigned int* counter = nullptr;  // blocks done, for the last-block scalar reductions
-  int red_blocks = 0;               // grid of the node kernels that reduce (8 CTAs per SM)
+  double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *b = nullptr;
+  float *r32 = nullptr, *p32 = nullptr, *q32 = nullptr, *e32 = nullptr;
+  double* part = nullptr;  // block partials [4][nblk]: the vector kernels' three, then <p, Ap>
+  int nsm = 0;
   int nblk = 0;
   double* scal = nullptr;  // device scalars
   double* hscal = nullptr; // pinned host mirror
@@ -111,7 +110,7 @@ __global__ void k_metric(int64_t total, const double* __restrict__ geo, double* 
 // Jacobi diagonal K_aa (unpinned), one thread per node over its elements in ascending order
 __global__ void k_diag(int n, const int32_t* __restrict__ n2e_ptr, const int32_t* __restrict__ n2e,
                        const double* __restrict__ geo, const DMat D, double* __restrict__ diag,
-                       float* __restrict__ diag32) {
+                       double* __restrict__ idiag, float* __restrict__ idiag32) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= n) return;
   double dsum = 0.0;
@@ -141,7 +140,8 @@ __global__ void k_diag(int n, const int32_t* __restrict__ n2e_ptr, const int32_t
     }
   }
   diag[row] = dsum;
-  diag32[row] = (float)dsum;
+  idiag[row] = 1.0 / dsum;
+  idiag32[row] = (float)(1.0 / dsum);
 }
 
 // element residuals of K x (x(pin) read as 0); skipped once the solve is done
@@ -318,39 +318,32 @@ __global__ void __launch_bounds__(64 * EPB, kRingCtas) k_lap_elem_async(int nele
 }
 
 
-// single-block fixed-order reductions of the partials and the CG scalars
+// single-block fixed-order reductions of the partials
 // mode 0: init  (part0 = ||r||^2 -> T1 and BNORM2, part1 = <r,z> -> Q1; done if ||b|| = 0)
-// mode 1: alpha (part0 = <p,Ap> -> Q2, alpha = Q1/Q2)
-// mode 2: update(part0 -> T1, part1 -> num, part2 -> Q1new; beta = num/Q1; Q1 = Q1new;
-//                iteration += 1; done if ||r|| < tol ||b|| or the iteration limit is reached)
 // mode 3: norm  (part0 -> T1)
-// modes 1 and 2 do nothing once done
 // Any block size up to 1024 threads; every thread of the block calls it.
 __device__ __forceinline__ void cg_scalars_block(int nblk, const double* __restrict__ part, int stride, int mode,
                                                  double* scal) {
-  __shared__ double sh[3][32];
-  const int np = mode == 2 ? 3 : (mode == 0 ? 2 : 1);
-  double v[3] = {0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-    for (int k = 0; k < np; ++k) v[k] += __ldcg(part + k * stride + b);
-  for (int k = 0; k < 3; ++k)
+  __shared__ double sh[2][32];
+  const int np = mode == 0 ? 2 : 1;
+  double v[2] = {0.0, 0.0};
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    v[0] += __ldcg(part + b);
+    if (np > 1) v[1] += __ldcg(part + stride + b);
+  }
+  for (int k = 0; k < 2; ++k)
     for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
   if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; ++k) sh[k][threadIdx.x >> 5] = v[k];
+    for (int k = 0; k < 2; ++k) sh[k][threadIdx.x >> 5] = v[k];
   __syncthreads();
   if (threadIdx.x == 0) {
-    double t[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < 3; ++k)
+    double t[2] = {0.0, 0.0};
+    for (int k = 0; k < 2; ++k)
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t[k] += sh[k][w];
     if (mode == 0) {
       scal[S_T1] = t[0]; scal[S_BNORM2] = t[0]; scal[S_Q1] = t[1];
       if (t[0] == 0.0) scal[S_DONE] = 1.0;
-    } else if (mode == 1) {
-      scal[S_Q2] = t[0]; scal[S_ALPHA] = scal[S_Q1] / t[0];
-    } else if (mode == 2) {
-      scal[S_T1] = t[0]; scal[S_NUM] = t[1]; scal[S_BETA] = t[1] / scal[S_Q1]; scal[S_Q1] = t[2];
-      scal[S_ITER] += 1.0;
-      if (sqrt(t[0]) < scal[S_TOL] * sqrt(scal[S_BNORM2]) || scal[S_ITER] >= scal[S_MAXIT]) scal[S_DONE] = 1.0;
     } else {
       scal[S_T1] = t[0];
     }
@@ -359,25 +352,36 @@ __device__ __forceinline__ void cg_scalars_block(int nblk, const double* __restr
 
 __global__ void __launch_bounds__(1024) k_cg_scalars(int nblk, const double* __restrict__ part, int stride,
                                                      int mode, double* scal) {
-  if ((mode == 1 || mode == 2) && scal[S_DONE] != 0.0) return;
   cg_scalars_block(nblk, part, stride, mode, scal);
 }
 
-// After a kernel's block partials: the last block to finish reduces them (cg_scalars_block in
-// the given mode) in a fixed order, so the CG scalars need no launch of their own.
-__device__ __forceinline__ void last_block_scalars(unsigned int* counter, const double* part, int stride, int mode,
-                                                   double* scal) {
-  __shared__ bool last;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+// The CG iteration's scalars are formed by the kernel that needs them: each of its blocks sums the
+// block partials of the kernel before in the same fixed order (a few hundred values from L2).  A last
+// block behind a fence and an atomic per block cost ~4 us at the end of each of the two kernels.  24^3,
+// FP64, per iteration: gather 9.2 -> 7.0 us, update 10.3 -> 4.8, p update 2.6 -> 4.4.
+// Sums NP partial columns over the block; every thread gets the totals.
+template <int NP>
+__device__ __forceinline__ void sum_partials(const double* __restrict__ part, int stride, int nblk, double (&t)[NP]) {
+  __shared__ double sh[NP][kBlock / 32];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) t[k] = 0.0;
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblk; b += kBlock)
+#pragma unroll
+    for (int k = 0; k < NP; ++k) t[k] += part[k * stride + b];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = t[k];
   }
   __syncthreads();
-  if (last) {
-    __threadfence();
-    cg_scalars_block(gridDim.x, part, stride, mode, scal);
-    if (threadIdx.x == 0) *counter = 0u;
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    t[k] = 0.0;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) t[k] += sh[k][w];
   }
+  __syncthreads();
 }
 
 template <int NP>
@@ -399,53 +403,69 @@ __device__ __forceinline__ void block_partials(double (&v)[NP], double* part, in
     }
 }
 
-// y = sum of the element residuals of each node, y(pin) = 0; partials of <x, y>
+// y = sum of the element residuals of each node, y(pin) = 0; partials of <x, y>.  Two nodes per trip:
+// a node is a chain of three loads (CSR range -> indices -> residuals), two run at once.
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_lap_gather(int n, int pin, const int32_t* __restrict__ n2e_ptr,
                                                       const int32_t* __restrict__ n2e, const T* __restrict__ rel,
                                                       const T* __restrict__ x, T* __restrict__ y,
-                                                      double* __restrict__ part, double* scal, unsigned int* counter) {
+                                                      double* __restrict__ part, const double* __restrict__ scal) {
   if (scal && scal[S_DONE] != 0.0) return;
   double v[1] = {0.0};
-  // grid-stride over the nodes: a grid of a few CTAs per SM keeps the partials (and the last
-  // block's reduction of them) short
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    T s = (T)0;
-    int c = n2e_ptr[i];
-    const int c1 = n2e_ptr[i + 1];
-    // up to kGather independent loads in flight (a hexahedral vertex has 8 elements), summed in
-    // ascending element order
-    for (; c < c1; c += kGather) {
-      int ix[kGather];
+  const int stride = gridDim.x * blockDim.x;
+  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 2 * stride) {
+    const int nd[2] = {i0, i0 + stride};
+    int c[2], e[2];
+    T xv[2], s[2] = {(T)0, (T)0};
 #pragma unroll
-      for (int u = 0; u < kGather; ++u) ix[u] = c + u < c1 ? n2e[c + u] : -1;
-      T v[kGather];
-#pragma unroll
-      for (int u = 0; u < kGather; ++u) v[u] = ix[u] >= 0 ? rel[ix[u]] : (T)0;
-#pragma unroll
-      for (int u = 0; u < kGather; ++u)
-        if (ix[u] >= 0) s += v[u];
+    for (int h = 0; h < 2; ++h) {
+      const bool in = nd[h] < n;
+      c[h] = in ? n2e_ptr[nd[h]] : 0;
+      e[h] = in ? n2e_ptr[nd[h] + 1] : 0;
+      xv[h] = in ? x[nd[h]] : (T)0;
     }
-    if (i == pin) s = (T)0;
-    y[i] = s;
-    v[0] += (double)x[i] * (double)s;
+    // up to kGather independent loads of each node in flight, summed in ascending element order
+    while (c[0] < e[0] || c[1] < e[1]) {
+      int ix[2][kGather];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < kGather; ++u) ix[h][u] = c[h] + u < e[h] ? n2e[c[h] + u] : -1;
+      T r[2][kGather];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < kGather; ++u) r[h][u] = ix[h][u] >= 0 ? rel[ix[h][u]] : (T)0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int u = 0; u < kGather; ++u)
+          if (ix[h][u] >= 0) s[h] += r[h][u];
+        c[h] += kGather;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (nd[h] < n) {
+        if (nd[h] == pin) s[h] = (T)0;
+        y[nd[h]] = s[h];
+        v[0] += (double)xv[h] * (double)s[h];
+      }
   }
   block_partials<1>(v, part, 0);
-  // inside CG (counter given): <p,Ap> and alpha = <r,z>/<p,Ap> by the last block (mode 1)
-  if (counter) last_block_scalars(counter, part, 0, 1, scal);
 }
 
 // r = b - Ax (ax may be null), z = r/M, p = z, x = 0 (if given); partials ||r||^2, <r,z>
 template <typename TV>
 __global__ void __launch_bounds__(kBlock) k_cg_init(int n, const TV* __restrict__ b, const TV* __restrict__ ax,
-                                                    const TV* __restrict__ M, TV* r, TV* z, TV* p, TV* x,
+                                                    const TV* __restrict__ iM, TV* r, TV* p, TV* x,
                                                     double* part, int stride) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double v[2] = {0.0, 0.0};
   if (i < n) {
     const TV ri = b[i] - (ax ? ax[i] : (TV)0);
-    const TV zi = ri / M[i];
-    r[i] = ri; z[i] = zi; p[i] = zi;
+    const TV zi = ri * iM[i];
+    r[i] = ri; p[i] = zi;
     if (x) x[i] = (TV)0;
     v[0] = (double)ri * (double)ri;
     v[1] = (double)ri * (double)zi;
@@ -453,79 +473,85 @@ __global__ void __launch_bounds__(kBlock) k_cg_init(int n, const TV* __restrict_
   block_partials<2>(v, part, stride);
 }
 
-// x += alpha p; r -= alpha q; z_old = z; z = r/M; partials ||r||^2, <r, z - z_old>, <r, z>
+// Nodes per thread and trip of the vector kernels, moved as 16-byte accesses (4- or 8-byte ones keep
+// too few bytes in flight)
+template <typename TV> struct CgVec;
+template <> struct CgVec<float> { using V = float4; static constexpr int K = 4; };
+template <> struct CgVec<double> { using V = double2; static constexpr int K = 2; };
 template <typename TV>
-__global__ void __launch_bounds__(kBlock) k_cg_update(int n, double* scal, TV* x, TV* r, TV* z,
-                                                      const TV* __restrict__ p, const TV* __restrict__ q,
-                                                      const TV* __restrict__ M, double* part, int stride,
-                                                      unsigned int* counter) {
+__device__ __forceinline__ void ldv(const TV* p, int t, TV (&o)[CgVec<TV>::K]) {
+  *reinterpret_cast<typename CgVec<TV>::V*>(o) = reinterpret_cast<const typename CgVec<TV>::V*>(p)[t];
+}
+template <typename TV>
+__device__ __forceinline__ void stv(TV* p, int t, const TV (&o)[CgVec<TV>::K]) {
+  reinterpret_cast<typename CgVec<TV>::V*>(p)[t] = *reinterpret_cast<const typename CgVec<TV>::V*>(o);
+}
+
+// alpha = <r,z> / <p,Ap>; x += alpha p; r -= alpha q; z = r/M; partials ||r||^2, <r, z - z_old>, <r, z>.
+// z is not stored: z_old is the old r times 1/M again, which saves two of the nine vectors the update
+// moved (and every division); the p update forms it once more from r.
+template <typename TV>
+__global__ void __launch_bounds__(kBlock) k_cg_update(int n, double* scal, const double* __restrict__ pq, int npq,
+                                                      TV* x, TV* r, const TV* __restrict__ p, const TV* __restrict__ q,
+                                                      const TV* __restrict__ iM, double* part, int stride) {
+  constexpr int K = CgVec<TV>::K;
   if (scal[S_DONE] != 0.0) return;
+  const double q1 = scal[S_Q1];
+  double t1[1];
+  sum_partials<1>(pq, 0, npq, t1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) scal[S_Q1OLD] = q1;  // the p update replaces Q1 while it reads this
   double v[3] = {0.0, 0.0, 0.0};
-  const TV alpha = (TV)scal[S_ALPHA];
-  auto one = [&](int i) {
-    x[i] = x[i] + alpha * p[i];
-    const TV ri = r[i] - alpha * q[i];
-    const TV zo = z[i];
-    const TV zi = ri / M[i];
-    r[i] = ri; z[i] = zi;
+  const TV alpha = (TV)(q1 / t1[0]);
+  auto one = [&](TV& xi, TV& ri, TV pi, TV qi, TV mi) {
+    xi = xi + alpha * pi;
+    const TV zo = ri * mi;
+    ri = ri - alpha * qi;
+    const TV zi = ri * mi;
     v[0] += (double)ri * (double)ri;
     v[1] += (double)ri * ((double)zi - (double)zo);
     v[2] += (double)ri * (double)zi;
   };
   const int gstride = gridDim.x * blockDim.x;
-  int i0 = 0;
-  if constexpr (sizeof(TV) == 4) {
-    // FP32 sweeps: four nodes per thread through 16-byte accesses (a 4-byte load per node keeps
-    // too few bytes in flight to reach the HBM rate)
-    const int n4 = n >> 2;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n4; t += gstride) {
-      float4 xv = reinterpret_cast<const float4*>(x)[t], pv = reinterpret_cast<const float4*>(p)[t];
-      float4 rv = reinterpret_cast<const float4*>(r)[t], qv = reinterpret_cast<const float4*>(q)[t];
-      float4 zv = reinterpret_cast<const float4*>(z)[t], mv = reinterpret_cast<const float4*>(M)[t];
-      float xa[4] = {xv.x, xv.y, xv.z, xv.w}, pa[4] = {pv.x, pv.y, pv.z, pv.w}, ra[4] = {rv.x, rv.y, rv.z, rv.w};
-      float qa[4] = {qv.x, qv.y, qv.z, qv.w}, za[4] = {zv.x, zv.y, zv.z, zv.w}, ma[4] = {mv.x, mv.y, mv.z, mv.w};
+  const int nv = n / K;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += gstride) {
+    __align__(16) TV xa[K], ra[K], pa[K], qa[K], ma[K];
+    ldv(x, t, xa); ldv(r, t, ra); ldv(p, t, pa); ldv(q, t, qa); ldv(iM, t, ma);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        xa[c] = xa[c] + alpha * pa[c];
-        const float ri = ra[c] - alpha * qa[c];
-        const float zo = za[c];
-        const float zi = ri / ma[c];
-        ra[c] = ri; za[c] = zi;
-        v[0] += (double)ri * (double)ri;
-        v[1] += (double)ri * ((double)zi - (double)zo);
-        v[2] += (double)ri * (double)zi;
-      }
-      reinterpret_cast<float4*>(x)[t] = make_float4(xa[0], xa[1], xa[2], xa[3]);
-      reinterpret_cast<float4*>(r)[t] = make_float4(ra[0], ra[1], ra[2], ra[3]);
-      reinterpret_cast<float4*>(z)[t] = make_float4(za[0], za[1], za[2], za[3]);
-    }
-    i0 = n4 << 2;
+    for (int c = 0; c < K; ++c) one(xa[c], ra[c], pa[c], qa[c], ma[c]);
+    stv(x, t, xa); stv(r, t, ra);
   }
-  for (int i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gstride) one(i);
+  for (int i = nv * K + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gstride) one(x[i], r[i], p[i], q[i], iM[i]);
   block_partials<3>(v, part, stride);
-  // beta, the iteration count and the stop test by the last block (mode 2)
-  last_block_scalars(counter, part, stride, 2, scal);
 }
 
+// beta = <r, z - z_old> / <r,z>_old; p = z + beta p, z = r/M; block 0 writes the iteration's scalars
+// and the stop test.  (A block that starts after that may see S_DONE and leave its part of p: the
+// solve is then over.)
 template <typename TV>
-__global__ void k_cg_pupdate(int n, const double* __restrict__ scal, const TV* __restrict__ z, TV* p) {
+__global__ void __launch_bounds__(kBlock) k_cg_pupdate(int n, double* scal, const double* __restrict__ part, int stride,
+                                                       int npart, const TV* __restrict__ r, const TV* __restrict__ iM,
+                                                       TV* p) {
+  constexpr int K = CgVec<TV>::K;
   if (scal[S_DONE] != 0.0) return;
-  const TV beta = (TV)scal[S_BETA];
-  if constexpr (sizeof(TV) == 4) {  // four nodes per thread, 16-byte accesses
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n4 = n >> 2;
-    if (t < n4) {
-      const float4 zv = reinterpret_cast<const float4*>(z)[t];
-      float4 pv = reinterpret_cast<float4*>(p)[t];
-      pv.x = zv.x + beta * pv.x; pv.y = zv.y + beta * pv.y; pv.z = zv.z + beta * pv.z; pv.w = zv.w + beta * pv.w;
-      reinterpret_cast<float4*>(p)[t] = pv;
-    }
-    const int i = (n4 << 2) + t;
-    if (t < (n & 3)) p[i] = z[i] + beta * p[i];
-  } else {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = z[i] + beta * p[i];
+  double t3[3];
+  sum_partials<3>(part, stride, npart, t3);
+  const double beta_d = t3[1] / scal[S_Q1OLD];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal[S_T1] = t3[0]; scal[S_NUM] = t3[1]; scal[S_BETA] = beta_d; scal[S_Q1] = t3[2];
+    const double it = scal[S_ITER] + 1.0;
+    scal[S_ITER] = it;
+    if (sqrt(t3[0]) < scal[S_TOL] * sqrt(scal[S_BNORM2]) || it >= scal[S_MAXIT]) scal[S_DONE] = 1.0;
   }
+  const TV beta = (TV)beta_d;
+  const int nv = n / K, gstride = gridDim.x * blockDim.x;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += gstride) {
+    __align__(16) TV ra[K], ma[K], pa[K];
+    ldv(r, t, ra); ldv(iM, t, ma); ldv(p, t, pa);
+#pragma unroll
+    for (int c = 0; c < K; ++c) pa[c] = ra[c] * ma[c] + beta * pa[c];
+    stv(p, t, pa);
+  }
+  for (int i = nv * K + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gstride) p[i] = r[i] * iM[i] + beta * p[i];
 }
 
 __global__ void k_cg_setup(double* scal, double tol, int max_iter) {
@@ -561,11 +587,17 @@ using namespace sod;
 using namespace sod::cg;
 
 static int node_grid(int64_t n) { return (int)((n + kBlock - 1) / kBlock); }
-// grid of the node kernels with reductions (grid-stride loops): a few CTAs per SM
-static int red_grid(const SodPoisson* P) { return std::min(P->nblk, P->red_blocks); }
+// Grid of the node kernels: at most `cap` CTAs per SM, the trips of the grid-stride loop shared out evenly
+// (a grid just below the work leaves most threads waiting for the few that take one trip more).  The
+// reducing ones stay at a few CTAs per SM, since every block of the next kernel sums their partials.
+static int node_blocks(const SodPoisson* P, int64_t groups, int cap) {
+  const int64_t most = (int64_t)cap * P->nsm, trips = (groups + most - 1) / most;
+  return (int)((groups + trips - 1) / trips);
+}
+static int gather_blocks(const SodPoisson* P) { return node_blocks(P, (P->n + 2 * kBlock - 1) / (2 * kBlock), 4); }
 
-// y = K x with <x, y> block partials (part[0..node_grid(n))); scal != null skips once done and
-// then also forms alpha (the CG iteration's scalars) in the gather's last block
+// y = K x with the block partials of <x, y> in the fourth column of part (gather_blocks of them);
+// scal != null skips once done
 template <typename T>
 static int lap_apply(SodPoisson* P, const T* x, T* y, double* scal, cudaStream_t st) {
   const SodMesh* m = P->mesh;
@@ -587,8 +619,8 @@ static int lap_apply(SodPoisson* P, const T* x, T* y, double* scal, cudaStream_t
     k_lap_elem<T><<<ngroups, 64 * EPB, 0, st>>>(E, P->pin, m->econn, met, *D, x, rel, scal);
   }
   SOD_CHECK_LAUNCH();
-  k_lap_gather<T><<<red_grid(P), kBlock, 0, st>>>((int)P->n, P->pin, m->n2e_ptr, m->n2e, rel, x, y, P->part, scal,
-                                                  scal ? P->counter : nullptr);
+  k_lap_gather<T><<<gather_blocks(P), kBlock, 0, st>>>((int)P->n, P->pin, m->n2e_ptr, m->n2e, rel, x, y,
+                                                       P->part + 3 * (size_t)P->nblk, scal);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
@@ -606,24 +638,25 @@ static int read_scalars(SodPoisson* P, cudaStream_t st) {
 
 template <typename TV>
 struct CgVecs {
-  const TV* M; TV *e, *r, *z, *p, *q;
+  const TV* iM; TV *e, *r, *p, *q;
 };
 
 // FP64: the solve's own vectors; FP32 sweep: its residual overwrites its right-hand side r32
 template <typename TV> static CgVecs<TV> vecs(SodPoisson* P);
-template <> CgVecs<double> vecs<double>(SodPoisson* P) { return {P->diag, P->x, P->r, P->z, P->p, P->q}; }
-template <> CgVecs<float> vecs<float>(SodPoisson* P) { return {P->diag32, P->e32, P->r32, P->z32, P->p32, P->q32}; }
+template <> CgVecs<double> vecs<double>(SodPoisson* P) { return {P->idiag, P->x, P->r, P->p, P->q}; }
+template <> CgVecs<float> vecs<float>(SodPoisson* P) { return {P->idiag32, P->e32, P->r32, P->p32, P->q32}; }
 
 // one CG iteration after the init (matvec, alpha, update, beta + stop test, p update)
 template <typename TV>
 static int cg_iteration(SodPoisson* P, const CgVecs<TV>& v, cudaStream_t st) {
   const int n = (int)P->n;
-  const int gb = node_grid(n);
-  if (int rc = lap_apply<TV>(P, v.p, v.q, P->scal, st)) return rc;  // + alpha
-  k_cg_update<TV><<<red_grid(P), kBlock, 0, st>>>(n, P->scal, v.e, v.r, v.z, v.p, v.q, v.M, P->part, P->nblk,
-                                                  P->counter);  // + beta and the stop test
+  const int64_t groups = (n + (int64_t)CgVec<TV>::K * kBlock - 1) / ((int64_t)CgVec<TV>::K * kBlock);
+  const int gu = node_blocks(P, groups, 4);
+  if (int rc = lap_apply<TV>(P, v.p, v.q, P->scal, st)) return rc;
+  k_cg_update<TV><<<gu, kBlock, 0, st>>>(n, P->scal, P->part + 3 * (size_t)P->nblk, gather_blocks(P), v.e, v.r, v.p, v.q,
+                                         v.iM, P->part, P->nblk);
   SOD_CHECK_LAUNCH();
-  k_cg_pupdate<TV><<<sizeof(TV) == 4 ? node_grid((n + 3) / 4) : gb, kBlock, 0, st>>>(n, P->scal, v.z, v.p);
+  k_cg_pupdate<TV><<<node_blocks(P, groups, 8), kBlock, 0, st>>>(n, P->scal, P->part, P->nblk, gu, v.r, v.iM, v.p);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
@@ -677,7 +710,7 @@ static int pcg(SodPoisson* P, const CgVecs<TV>& v, const TV* rhs, int max_iter, 
   if (int rc = batch_graph<TV>(P, &exec, &nk)) return rc;
   k_cg_setup<<<1, 1, 0, st>>>(P->scal, tol, max_iter);
   SOD_CHECK_LAUNCH();
-  k_cg_init<TV><<<gb, kBlock, 0, st>>>(n, rhs, (const TV*)nullptr, v.M, v.r, v.z, v.p, v.e, P->part, P->nblk);
+  k_cg_init<TV><<<gb, kBlock, 0, st>>>(n, rhs, (const TV*)nullptr, v.iM, v.r, v.p, v.e, P->part, P->nblk);
   SOD_CHECK_LAUNCH();
   if (int rc = scalars(P, gb, 0, st)) return rc;
   if (int rc = read_scalars(P, st)) return rc;
@@ -704,8 +737,8 @@ void sod_poisson_destroy(SodPoisson* P) {
   if (!P) return;
   for (cudaGraphExec_t& g : P->batch)
     if (g) cudaGraphExecDestroy(g);
-  void* ptrs[] = {P->met, P->met32, P->diag, P->diag32, P->rel, P->x, P->r, P->p, P->q, P->z, P->b,
-                  P->r32, P->p32, P->q32, P->z32, P->e32, P->part, P->scal, P->counter};
+  void* ptrs[] = {P->met, P->met32, P->diag, P->idiag, P->idiag32, P->rel, P->x, P->r, P->p, P->q, P->b,
+                  P->r32, P->p32, P->q32, P->e32, P->part, P->scal};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (P->hscal) cudaFreeHost(P->hscal);
@@ -738,13 +771,12 @@ int sod_poisson_create(SodMesh* m, SodPoisson** out) {
   PALLOC(P->met32, sizeof(float) * NMET * NN * E);
   PALLOC(P->rel, sizeof(double) * NN * E);
   PALLOC(P->diag, sizeof(double) * N);
-  PALLOC(P->diag32, sizeof(float) * N);
-  for (double** v : {&P->x, &P->r, &P->p, &P->q, &P->z, &P->b}) PALLOC(*v, sizeof(double) * N);
-  for (float** v : {&P->r32, &P->p32, &P->q32, &P->z32, &P->e32}) PALLOC(*v, sizeof(float) * N);
-  PALLOC(P->part, sizeof(double) * 3 * P->nblk);
+  PALLOC(P->idiag, sizeof(double) * N);
+  PALLOC(P->idiag32, sizeof(float) * N);
+  for (double** v : {&P->x, &P->r, &P->p, &P->q, &P->b}) PALLOC(*v, sizeof(double) * N);
+  for (float** v : {&P->r32, &P->p32, &P->q32, &P->e32}) PALLOC(*v, sizeof(float) * N);
+  PALLOC(P->part, sizeof(double) * 4 * P->nblk);
   PALLOC(P->scal, sizeof(double) * S_COUNT);
-  PALLOC(P->counter, sizeof(unsigned int));
-  if (cudaMemset(P->counter, 0, sizeof(unsigned int)) != cudaSuccess) return fail("counter");
 #undef PALLOC
   if (cudaMallocHost(&P->hscal, sizeof(double) * S_COUNT) != cudaSuccess) return fail("hscal");
   {
@@ -761,10 +793,10 @@ int sod_poisson_create(SodMesh* m, SodPoisson** out) {
                                                            LapRing<float, NSTAGE>::kBytes));
     P->ring_grid[0] = nsm * b64;
     P->ring_grid[1] = nsm * b32;
-    P->red_blocks = 8 * nsm;
+    P->nsm = nsm;
   }
   k_metric<<<1184, 256>>>(E * NN, m->geo64, P->met, P->met32);
-  k_diag<<<node_grid(N), kBlock>>>((int)N, m->n2e_ptr, m->n2e, m->geo64, m->D, P->diag, P->diag32);
+  k_diag<<<node_grid(N), kBlock>>>((int)N, m->n2e_ptr, m->n2e, m->geo64, m->D, P->diag, P->idiag, P->idiag32);
   g_launches.fetch_add(2);
   cudaError_t err = cudaDeviceSynchronize();
   if (err == cudaSuccess) err = cudaGetLastError();
@@ -806,7 +838,7 @@ int sod_conjgrad_pressure(SodPoisson* P, const double* Rp0, double* R, int max_i
     if (rc) return rc;
   } else {
     // FP64 residual iterative refinement around FP32 Jacobi-PCG sweeps
-    k_cg_init<double><<<gb, kBlock, 0, st>>>(n, P->b, (const double*)nullptr, P->diag, P->r, P->z, P->p, P->x,
+    k_cg_init<double><<<gb, kBlock, 0, st>>>(n, P->b, (const double*)nullptr, P->idiag, P->r, P->p, P->x,
                                              P->part, P->nblk);
     SOD_CHECK_LAUNCH();
     if (int rc = scalars(P, gb, 0, st)) return rc;
@@ -827,7 +859,7 @@ int sod_conjgrad_pressure(SodPoisson* P, const double* Rp0, double* R, int max_i
       SOD_CHECK_LAUNCH();
       // r = b - A x in FP64, ||r||^2
       if (int rc2 = lap_apply<double>(P, P->x, P->q, nullptr, st)) return rc2;
-      k_cg_init<double><<<gb, kBlock, 0, st>>>(n, P->b, P->q, P->diag, P->r, P->z, P->p, (double*)nullptr, P->part,
+      k_cg_init<double><<<gb, kBlock, 0, st>>>(n, P->b, P->q, P->idiag, P->r, P->p, (double*)nullptr, P->part,
                                                P->nblk);
       SOD_CHECK_LAUNCH();
       if (int rc3 = scalars(P, gb, 3, st)) return rc3;
