@@ -4,11 +4,12 @@
 //
 // The boundary nodes are compacted once (sod_mesh_set_boundaries) into an ascending list with
 // their code, lnbn node, normal and buffer velocity; every kernel here runs one thread per
-// boundary node.  temporary_bc_routine_dirichlet_prim is two kernels: k_bc_gather copies the
-// state of every boundary node's lnbn node first (the reference's first loop), so a boundary
-// node whose lnbn node is itself on a boundary reads the value from before the routine, as
-// there; k_bc_apply forms the lnbn node's velocity and pressure and overwrites the boundary
-// node by code.
+// boundary node.  temporary_bc_routine_dirichlet_prim: k_bc_apply forms the lnbn node's velocity and
+// pressure and overwrites the boundary node by code.  Only the far-field code uses the lnbn node's
+// state.  When a far-field node's lnbn node is itself on a boundary, k_bc_gather copies the state of
+// every lnbn node first (the reference's first loop), so that it is the value from before the routine;
+// otherwise no lnbn node that is read changes, k_bc_apply reads the state itself, and the copy (a
+// launch per stage, ~3 us with its gap, on 15^3 elements) is left out.
 //
 // Inside a step the stage state is formed by the gather kernel of the previous stage (stage
 // 1: a copy of the state) and the routine runs on it before the element kernels evaluate its
@@ -57,7 +58,8 @@ struct ApplyArgs {
   const int32_t* code;
   const double* normal;  // [3][nb]
   const double* ubuf;    // [3][nb]
-  const double* aux2;    // [5][nb]
+  const double* aux2;    // [5][nb] state of the lnbn nodes (k_bc_gather), or null: read it from the state
+  const int32_t* nbr;    // lnbn node of each
   double *rho, *q, *E;   // state updated in place (node-indexed)
   const double* uold_b;  // slip branch velocity per boundary node [3][nb], or
   const double* uold_n;  // per node (npoin,3); both null: zero
@@ -174,9 +176,19 @@ __global__ void __launch_bounds__(kBlock) k_bc_apply(const ApplyArgs a) {
   const size_t n = (size_t)a.node[b];
   const int c = a.code[b];
   double own[5] = {a.rho[n], a.q[n], a.q[n + N], a.q[n + 2 * N], a.E[n]};
-  double nbv[5];
+  double nbv[5] = {1.0, 0.0, 0.0, 0.0, 1.0};  // not used by the other codes
+  if (c == kFarField) {
+    if (a.aux2) {
 #pragma unroll
-  for (int f = 0; f < 5; ++f) nbv[f] = a.aux2[f * nb + b];
+      for (int f = 0; f < 5; ++f) nbv[f] = a.aux2[f * nb + b];
+    } else {
+      const size_t s = (size_t)a.nbr[b];
+      nbv[0] = a.rho[s];
+#pragma unroll
+      for (int f = 0; f < 3; ++f) nbv[1 + f] = a.q[s + f * N];
+      nbv[4] = a.E[s];
+    }
+  }
   double uo[3] = {0.0, 0.0, 0.0};
   if (a.uold_b) {
 #pragma unroll
@@ -587,6 +599,9 @@ __global__ void __launch_bounds__(kBlock) k_eta_final(int nblk, int npoin, int n
 
 static int grid_of(int n) { return (n + kBlock - 1) / kBlock; }
 
+// a far-field node's lnbn node lies on a boundary: its state has to be kept from before the routine
+static bool copies_lnbn(const SodMesh* m) { return m->bc.nff > 0 && m->bc.ff_nbr_on_boundary; }
+
 static ApplyArgs base_args(SodMesh* m) {
   ApplyArgs a{};
   a.nb = m->bc.nb;
@@ -595,7 +610,8 @@ static ApplyArgs base_args(SodMesh* m) {
   a.code = m->bc.code;
   a.normal = m->bc.normal;
   a.ubuf = m->bc.ubuf;
-  a.aux2 = m->bc.aux2;
+  a.aux2 = copies_lnbn(m) ? m->bc.aux2 : nullptr;
+  a.nbr = m->bc.nbr;
   a.gamma = m->prm.gamma;
   a.Rgas = m->prm.Rgas;
   a.p = m->bc.prm;
@@ -603,6 +619,7 @@ static ApplyArgs base_args(SodMesh* m) {
 }
 
 static int gather(SodMesh* m, const double* rho, const double* q, const double* E, cudaStream_t st) {
+  if (!copies_lnbn(m)) return SOD_OK;
   k_bc_gather<<<grid_of(m->bc.nb), kBlock, 0, st>>>(m->bc.nb, m->bc.nbr, rho, q, E, (size_t)m->npoin, m->bc.aux2);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
@@ -703,6 +720,7 @@ void bc_free(SodMesh* m) {
 }
 
 int bc_snapshot_u(SodMesh* m, const double* u, cudaStream_t st) {
+  if (!m->bc.has_slip) return SOD_OK;  // only the slip codes read it
   bcd::k_bc_snapshot<<<bcd::grid_of(m->bc.nb), bcd::kBlock, 0, st>>>(m->bc.nb, m->bc.node, u, (size_t)m->npoin,
                                                                       m->bc.u_final);
   SOD_CHECK_LAUNCH();

@@ -636,6 +636,18 @@ __global__ void __launch_bounds__(256) k_member_eta(const int32_t* __restrict__ 
   done[mbr] = 0u;
 }
 
+// the first stage state of a step with boundaries or a buffer zone: (rho, q, E) as [5][N]
+__global__ void __launch_bounds__(256) k_copy_state(int64_t N, const double* __restrict__ rho,
+                                                    const double* __restrict__ q, const double* __restrict__ E,
+                                                    double* __restrict__ y) {
+  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  y[n] = rho[n];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) y[(1 + c) * N + n] = q[c * N + n];
+  y[4 * N + n] = E[n];
+}
+
 // Reta scratch when the caller passes none
 static double* reta_scratch(SodMesh* m) {
   // the FP64 rsum eta column, dead after stage 4 reads it (the mixed path's FP32 accumulators
@@ -727,9 +739,8 @@ int run_step(SodMesh* m, SodState* s, const double* dt_dev, double* dt_next, boo
     double* yin = (stage_store && stage >= 2) ? stage_store + (size_t)(stage - 2) * 5 * N : m->buf.ys;
     if (pre && stage == 1) {
       // the first stage state is the state itself with the routines applied to a copy
-      SOD_CUDA(cudaMemcpyAsync(yin, s->rho, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
-      SOD_CUDA(cudaMemcpyAsync(yin + N, s->q, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, st));
-      SOD_CUDA(cudaMemcpyAsync(yin + 4 * N, s->E, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
+      k_copy_state<<<(unsigned)((N + 255) / 256), 256, 0, st>>>((int64_t)N, s->rho, s->q, s->E, yin);
+      SOD_CHECK_LAUNCH();
       rc = pre_stage(yin, 1);
       if (rc) return rc;
     }
@@ -755,7 +766,8 @@ int run_step(SodMesh* m, SodState* s, const double* dt_dev, double* dt_next, boo
     g.pr = s->pr; g.Tem = s->Tem; g.e_int = s->e_int; g.eta = s->eta; g.csound = s->csound;
     g.machno = s->machno; g.mu_fluid = s->mu_fluid; g.Reta = loc.Reta; g.mu_factor = s->mu_factor;
     g.node_member = m->nmember > 0 ? m->node_member : nullptr;
-    g.member_reduce = m->nmember > 0 ? 1 : 0;
+    // (after boundary conditions or a buffer zone the entropy sums are formed from the changed state)
+    g.member_reduce = (m->nmember > 0 || pre) ? 1 : 0;
     if (stage_store && stage < 4) g.ys = stage_store + (size_t)(stage - 1) * 5 * N;
     if (ev) cudaEventRecord(ev[2 * (3 + stage)], st);
     rc = launch_gather(m, mixed, stage, g, st);
