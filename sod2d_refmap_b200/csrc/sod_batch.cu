@@ -211,14 +211,11 @@ int sod_batch_set_member(SodBatch* B, int member, const SodState* h) {
   SOD_CUDA(cudaMemcpy(B->st.rho + no, h->rho, 8 * Ni, cudaMemcpyHostToDevice));
   SOD_CUDA(cudaMemcpy(B->st.E + no, h->E, 8 * Ni, cudaMemcpyHostToDevice));
   SOD_CUDA(cudaMemcpy(B->st.mu_factor + no, h->mu_factor, 8 * Ni, cudaMemcpyHostToDevice));
-  for (int c = 0; c < 3; ++c) {
-    SOD_CUDA(cudaMemcpy(B->st.q + c * N + no, h->q + c * Ni, 8 * Ni, cudaMemcpyHostToDevice));
-    if (h->u) SOD_CUDA(cudaMemcpy(B->st.u + c * N + no, h->u + c * Ni, 8 * Ni, cudaMemcpyHostToDevice));
-  }
+  SOD_CUDA(cudaMemcpy2D(B->st.q + no, 8 * N, h->q, 8 * Ni, 8 * Ni, 3, cudaMemcpyHostToDevice));
+  if (h->u) SOD_CUDA(cudaMemcpy2D(B->st.u + no, 8 * N, h->u, 8 * Ni, 8 * Ni, 3, cudaMemcpyHostToDevice));
   if (h->csound) SOD_CUDA(cudaMemcpy(B->st.csound + no, h->csound, 8 * Ni, cudaMemcpyHostToDevice));
   if (h->mu_fluid) SOD_CUDA(cudaMemcpy(B->st.mu_fluid + no, h->mu_fluid, 8 * Ni, cudaMemcpyHostToDevice));
-  for (int a = 0; a < NN; ++a)
-    SOD_CUDA(cudaMemcpy(B->st.mu_e + a * E + eo, h->mu_e + a * Ei, 8 * Ei, cudaMemcpyHostToDevice));
+  SOD_CUDA(cudaMemcpy2D(B->st.mu_e + eo, 8 * E, h->mu_e, 8 * Ei, 8 * Ei, NN, cudaMemcpyHostToDevice));
   return SOD_OK;
 }
 
@@ -233,13 +230,10 @@ int sod_batch_get_member(SodBatch* B, int member, SodState* h) {
       {h->machno, B->st.machno}, {h->mu_fluid, B->st.mu_fluid}, {h->Reta, B->st.Reta}};
   for (auto& f : sc)
     if (f.hst) SOD_CUDA(cudaMemcpy(f.hst, f.dev + no, 8 * Ni, cudaMemcpyDeviceToHost));
-  for (int c = 0; c < 3; ++c) {
-    if (h->q) SOD_CUDA(cudaMemcpy(h->q + c * Ni, B->st.q + c * N + no, 8 * Ni, cudaMemcpyDeviceToHost));
-    if (h->u) SOD_CUDA(cudaMemcpy(h->u + c * Ni, B->st.u + c * N + no, 8 * Ni, cudaMemcpyDeviceToHost));
-  }
-  if (h->mu_e)
-    for (int a = 0; a < NN; ++a)
-      SOD_CUDA(cudaMemcpy(h->mu_e + a * Ei, B->st.mu_e + a * E + eo, 8 * Ei, cudaMemcpyDeviceToHost));
+  // a member's columns as one strided copy each (a copy per column of mu_e was 64 synchronous calls)
+  if (h->q) SOD_CUDA(cudaMemcpy2D(h->q, 8 * Ni, B->st.q + no, 8 * N, 8 * Ni, 3, cudaMemcpyDeviceToHost));
+  if (h->u) SOD_CUDA(cudaMemcpy2D(h->u, 8 * Ni, B->st.u + no, 8 * N, 8 * Ni, 3, cudaMemcpyDeviceToHost));
+  if (h->mu_e) SOD_CUDA(cudaMemcpy2D(h->mu_e, 8 * Ei, B->st.mu_e + eo, 8 * E, 8 * Ei, NN, cudaMemcpyDeviceToHost));
   return SOD_OK;
 }
 
