@@ -32,9 +32,9 @@
 // ^ marks contravariant fluxes.  Every field is held as its deviation from an element reference
 // (node 0, in FP64, before the FP32 cast); p from one that is affine in xi.
 //
-// Measured at 64^3 (262,144 elements, one launch): 0.826 ms, 1.254 ms with the 12 gradient fields
+// Measured at 64^3 (262,144 elements, one launch): 0.801 ms, 1.254 ms with the 12 gradient fields
 // and 25 staged-factor products of the quartets formed one by one.  Bounded by latency at 20
-// resident warps per SM with the L1 data pipe ~75% and the issue slots ~60% busy; HBM floor 0.24 ms.
+// resident warps per SM with the L1 data pipe ~70% and the issue slots ~55% busy; HBM floor 0.24 ms.
 //
 // Precision: div u is the one sum whose terms (the velocity gradients) cancel by orders of
 // magnitude, and it multiplies rho, H and eta, so its line sums and fold run in FP64 (45 FP64
@@ -58,7 +58,7 @@ constexpr int NSLOT = NA + NU + NP2;
 // doubles per element ahead of the slots: rho, u, h, k, T of node 0; p of the nodes (0,0,0), (3,0,0),
 // (0,3,0), (0,0,3); log p and log rho of node 0; then FP32 references (8 floats) and the slopes of p (3)
 constexpr int R_P = 7, R_LOG = R_P + 4, R_F32 = R_LOG + 3, NREF = R_F32 + 6;
-constexpr int NDTAB = 48;  // doubles per CTA: D and D^T as (v, v) float2 pairs, then D; rows of 4
+constexpr int NDTAB = 32;  // doubles per CTA: D and D^T in FP32, then D; rows of 4
 
 __host__ __device__ constexpr size_t smem_bytes(int epb) {
   return sizeof(double) * (NDTAB + (size_t)epb * NREF) + sizeof(float2) * (size_t)epb * NSLOT * FSTRIDE;
@@ -93,11 +93,11 @@ __device__ __forceinline__ float2 divT2(const float2* fx, const float2* fy, cons
   return ADD2(ADD2(s, t), u);
 }
 
-// a table row of 4 (v, v) pairs
-__device__ __forceinline__ void load_row(const float2* tab, int x, float2* w) {
-  const float4 a = *reinterpret_cast<const float4*>(tab + 4 * x), b = *reinterpret_cast<const float4*>(tab + 4 * x + 2);
-  w[0] = make_float2(a.x, a.y); w[1] = make_float2(a.z, a.w);
-  w[2] = make_float2(b.x, b.y); w[3] = make_float2(b.z, b.w);
+// A table row as 4 (v, v) pairs, doubled in registers: doubled rows in shared memory cost 24 more
+// wavefronts per element (0.831 against 0.801 ms at 64^3).
+__device__ __forceinline__ void load_row(const float* tab, int x, float2* w) {
+  const float4 a = *reinterpret_cast<const float4*>(tab + 4 * x);
+  w[0] = F2(a.x); w[1] = F2(a.y); w[2] = F2(a.z); w[3] = F2(a.w);
 }
 
 // Resident 64-thread element groups per SM the register budget must allow.  Measured at 64^3 (one
@@ -111,8 +111,8 @@ __device__ __forceinline__ void load_row(const float2* tab, int x, float2* w) {
 // TOTH: flag_total_enthalpy (energy convection of full_convec_ijk_H)
 template <int EPB, bool TOTH>
 __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsigned char* smem_raw) {
-  float2* dtab = reinterpret_cast<float2*>(smem_raw);   // D rows, then D^T rows
-  double* dtab64 = reinterpret_cast<double*>(smem_raw) + 32;
+  float* dtab = reinterpret_cast<float*>(smem_raw);   // D rows, then D^T rows
+  double* dtab64 = reinterpret_cast<double*>(smem_raw) + 16;
   double* refs_all = reinterpret_cast<double*>(smem_raw) + NDTAB;
   float2* buf_all = reinterpret_cast<float2*>(refs_all + EPB * NREF);
   const int tid = threadIdx.x;
@@ -148,7 +148,7 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
   const float gpv = geo[9 * NN + d];
   if (tid < 32) {
     const int r = (tid >> 2) & 3, c = tid & 3;
-    dtab[tid] = F2(tid < 16 ? a.Df[r][c] : a.Df[c][r]);
+    dtab[tid] = tid < 16 ? a.Df[r][c] : a.Df[c][r];
     if (tid < 16) dtab64[tid] = a.D.d[r][c];
   }
   // one FP64 reciprocal serves every division of the EOS (the deviations below need FP64)
