@@ -137,11 +137,15 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
   // ---------------- convection and pressure: both roles of every line pair ----------------
   double rb = 0.0, Hb = 0.0, pb = 0.0;
   double ub[3] = {0.0, 0.0, 0.0};
+  // D along the seed lines of the energy and momentum (the adjoint of pass 2's D^T), back to physical
+  // components: adjoints of tau u and tau, gpvol He(r,:) . (D S)
+  double tUb[3] = {0.0, 0.0, 0.0};
+  double taub[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
   {
     double X1 = 0.0, gb = 0.0;
 #pragma unroll
     for (int dir = 0; dir < 3; ++dir) {
-      double w1[4], w2[4], Y1 = 0.0;
+      double w1[4], w2[4], Y1 = 0.0, l1 = 0.0, lo[3] = {0.0, 0.0, 0.0};
       load4(dtab + 4 * row[dir], w1);
       load4(dtab + 16 + 4 * row[dir], w2);
 #pragma unroll
@@ -180,6 +184,16 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
 #pragma unroll
         for (int c = 0; c < 3; ++c) ub[c] += x2 * ol[c] + y2 * gl[c];
         pb += w2[m] * (gl[0] * ol[0] + gl[1] * ol[1] + gl[2] * ol[2]);
+        l1 += w1[m] * el;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) lo[c] += w1[m] * ol[c];
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const double hr = G[3 * r + dir];
+        tUb[r] += hr * l1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) taub[c][r] += hr * lo[c];
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) ub[c] += Y1 * G[3 * c + dir];
@@ -198,7 +212,9 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
   // ---------------- forward gradients, and D along the seed lines ----------------
   pass_fence();
   const double igpv = 1.0 / Ge[9 * NN + d];  // G holds gpvol He; the forward gradients want He
+  // (with the other two seeds, of grad rho and grad T)
   double gU[3][3];
+  double gRhob[3] = {0.0, 0.0, 0.0}, gTb[3] = {0.0, 0.0, 0.0};
   {
     double gRho[3] = {0.0, 0.0, 0.0}, gT[3] = {0.0, 0.0, 0.0};
 #pragma unroll
@@ -209,12 +225,14 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
     for (int dir = 0; dir < 3; ++dir) {
       double w1[4];
       load4(dtab + 4 * row[dir], w1);
-      double lr = 0.0, lT = 0.0, lu[3] = {0.0, 0.0, 0.0};
+      double lr = 0.0, lT = 0.0, lu[3] = {0.0, 0.0, 0.0}, l0 = 0.0, l2 = 0.0;
 #pragma unroll
       for (int m = 0; m < NP1; ++m) {
         const double* f = sm + line[dir] + m * stride[dir];
         lr += w1[m] * f[F_RHO * FSTRIDE];
         lT += w1[m] * f[F_T * FSTRIDE];
+        l0 += w1[m] * f[W_NU * FSTRIDE];
+        l2 += w1[m] * f[W_KE * FSTRIDE];
 #pragma unroll
         for (int c = 0; c < 3; ++c) lu[c] += w1[m] * f[(F_U0 + c) * FSTRIDE];
       }
@@ -223,6 +241,8 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
         const double hr = G[3 * r + dir];
         gRho[r] += hr * lr;
         gT[r] += hr * lT;
+        gRhob[r] += hr * l0;
+        gTb[r] += hr * l2;
 #pragma unroll
         for (int c = 0; c < 3; ++c) gU[c][r] += hr * lu[c];
       }
@@ -238,35 +258,6 @@ __global__ void __launch_bounds__(64, SOD_VJP_MIN_BLOCKS) k_rhs_vjp(const VjpArg
     for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int r = 0; r < 3; ++r) gU[c][r] *= igpv;
-  }
-  pass_fence();
-  // adjoints of the contravariant fluxes (the adjoint of D^T is D along lines) back to the fluxes'
-  // physical components: Vb_r = gpvol He(r,:) . (D S_v)
-  double gRhob[3] = {0.0, 0.0, 0.0}, gTb[3] = {0.0, 0.0, 0.0}, tUb[3] = {0.0, 0.0, 0.0};
-  double taub[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-#pragma unroll
-  for (int dir = 0; dir < 3; ++dir) {
-    double w1[4];
-    load4(dtab + 4 * row[dir], w1);
-    double l0 = 0.0, l1 = 0.0, l2 = 0.0, lo[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int m = 0; m < NP1; ++m) {
-      const double* f = sm + line[dir] + m * stride[dir];
-      l0 += w1[m] * f[W_NU * FSTRIDE];
-      l1 += w1[m] * f[W_E * FSTRIDE];
-      l2 += w1[m] * f[W_KE * FSTRIDE];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) lo[c] += w1[m] * f[(W_O0 + c) * FSTRIDE];
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const double hr = G[3 * r + dir];
-      gRhob[r] += hr * l0;
-      tUb[r] += hr * l1;
-      gTb[r] += hr * l2;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) taub[c][r] += hr * lo[c];
-    }
   }
   // tauU_r = sum_c tau_rc u_c;  tau_rc = (mu_fgp+mue)(du_r/dx_c + du_c/dx_r) - delta_rc mu_fgp 2/3 div u,
   // mu_fgp = muf + rho musgs
