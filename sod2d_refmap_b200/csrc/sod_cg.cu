@@ -21,11 +21,11 @@
 //
 // The Jacobi diagonal is eval_laplacian_diag (mod_operators.f90:417-461): the unpinned K_aa.
 //
-// conjGrad_pressure_incomp (mod_solver_incomp.f90:247-434) runs as: product + <p,Ap>, whose
-// last block forms alpha; fused x/r/z update with ||r||^2, <r,z-z_old>, <r,z>, whose last block
-// forms beta and the stop test ||r|| < tol ||r0|| (:393); p update: four launches per iteration.  The stop test, the iteration counter and
-// a done flag live on the device, so iterations are replayed in CUDA-graph batches of kBatch
-// and the host reads the scalars once per batch; every kernel of an iteration after the
+// conjGrad_pressure_incomp (mod_solver_incomp.f90:247-434) runs as: product with the block partials of
+// <p,Ap>; x/r update, which forms alpha from them, with the partials of ||r||^2, <r,z-z_old>, <r,z>;
+// p update, which forms beta and the stop test ||r|| < tol ||r0|| (:393): four launches per iteration.
+// The iteration counter and a done flag live on the device, so iterations are replayed in CUDA-graph
+// batches of kBatch and the host reads the scalars once per batch; every kernel of an iteration after the
 // converged one returns at once, so the iterate and the count are those of a host-tested
 // loop.  mixed != 0 runs FP32 CG sweeps (FP32 metric and vectors) inside FP64 residual
 // iterative refinement.
@@ -47,7 +47,7 @@ constexpr int kBatch = 16;  // CG iterations per graph replay
 
 // device scalar slots
 enum {
-  S_Q1 = 0, S_Q2, S_T1, S_NUM, S_ALPHA, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD, S_COUNT
+  S_Q1 = 0, S_T1, S_NUM, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD, S_COUNT
 };
 
 template <typename T>

@@ -19,10 +19,6 @@
 // With eta = (rho L_r + lam) / (gamma - 1), L = log p - gamma log rho, L_r its value at the element's
 // node 0 and lam = rho (L - L_r), the entropy residual is (L_r Rm + the same functional of lam) /
 // (gamma - 1), so lam (small) is differentiated and L_r enters once, at the end.
-// (flag_total_enthalpy, full_convec_ijk_H: 1/2 sum D (G_x + G_m)(V_x + V_m) with G = rho H, and
-// dG = rho dH + H drho + drho dH).  So one pass over the 12 line points of 4 slots serves the
-// gradients and every product, with no products staged, none of the q, rho H, h and k
-// derivatives formed, and the metric folded into V before the sums instead of after them.
 //
 // Nodal fields are staged in shared memory as float2 pairs: one 8-byte shared load and one packed
 // __ffma2_rn serve two fields, and the xi-lines are read as 16-byte loads.  Slots:
