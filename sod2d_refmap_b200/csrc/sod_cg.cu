@@ -47,7 +47,9 @@ constexpr int kBatch = 16;  // CG iterations per graph replay
 
 // device scalar slots
 enum {
-  S_Q1 = 0, S_T1, S_NUM, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD, S_COUNT
+  S_Q1 = 0, S_T1, S_NUM, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD,
+  S_SKIP,  // S_DONE as the update kernel found it: the p update stores S_DONE, so none of its threads reads it
+  S_COUNT
 };
 
 template <typename T>
@@ -495,11 +497,14 @@ __global__ void __launch_bounds__(kBlock) k_cg_update(int n, double* scal, const
                                                       TV* x, TV* r, const TV* __restrict__ p, const TV* __restrict__ q,
                                                       const TV* __restrict__ iM, double* part, int stride) {
   constexpr int K = CgVec<TV>::K;
-  if (scal[S_DONE] != 0.0) return;
-  const double q1 = scal[S_Q1];
+  const double done = scal[S_DONE], q1 = scal[S_Q1];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal[S_SKIP] = done;
+    scal[S_Q1OLD] = q1;  // the p update replaces Q1 while it reads this
+  }
+  if (done != 0.0) return;
   double t1[1];
   sum_partials<1>(pq, 0, npq, t1);
-  if (blockIdx.x == 0 && threadIdx.x == 0) scal[S_Q1OLD] = q1;  // the p update replaces Q1 while it reads this
   double v[3] = {0.0, 0.0, 0.0};
   const TV alpha = (TV)(q1 / t1[0]);
   auto one = [&](TV& xi, TV& ri, TV pi, TV qi, TV mi) {
@@ -525,14 +530,14 @@ __global__ void __launch_bounds__(kBlock) k_cg_update(int n, double* scal, const
 }
 
 // beta = <r, z - z_old> / <r,z>_old; p = z + beta p, z = r/M; block 0 writes the iteration's scalars
-// and the stop test.  (A block that starts after that may see S_DONE and leave its part of p: the
-// solve is then over.)
+// and the stop test.  No thread reads a slot that block 0 writes (only block 0 its own iteration count):
+// the early return must be the same for a whole block, which has barriers after it.
 template <typename TV>
 __global__ void __launch_bounds__(kBlock) k_cg_pupdate(int n, double* scal, const double* __restrict__ part, int stride,
                                                        int npart, const TV* __restrict__ r, const TV* __restrict__ iM,
                                                        TV* p) {
   constexpr int K = CgVec<TV>::K;
-  if (scal[S_DONE] != 0.0) return;
+  if (scal[S_SKIP] != 0.0) return;
   double t3[3];
   sum_partials<3>(part, stride, npart, t3);
   const double beta_d = t3[1] / scal[S_Q1OLD];
