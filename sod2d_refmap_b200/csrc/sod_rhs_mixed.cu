@@ -23,20 +23,22 @@
 // Nodal fields are staged in shared memory as float2 pairs: one 8-byte shared load and one packed
 // __ffma2_rn serve two fields, and the xi-lines are read as 16-byte loads.  Slots:
 //   (u0,u1) (u2,H) (rho,lam) (p,T)                                 the nodal fields
-//   u0 u1 u2 in FP64                                               for div u
+//   u0 u1 u2 in FP64                                               for the velocity gradients
 //   (gradRho^,tauU^)x3 (gradT^,tauX^)x3 (tauY^,tauZ^)x3            pass 2, one slot per direction
 // ^ marks contravariant fluxes.  Every field is held as its deviation from an element reference
-// (node 0, in FP64, before the FP32 cast); p from one that is affine in xi.
+// (node 0, in FP64, before the FP32 cast); p and T from one that is affine in xi.
 //
-// Measured at 64^3 (262,144 elements, one launch): 0.801 ms, 1.254 ms with the 12 gradient fields
+// Measured at 64^3 (262,144 elements, one launch): 0.822 ms, 1.254 ms with the 12 gradient fields
 // and 25 staged-factor products of the quartets formed one by one.  Bounded by latency at 20
 // resident warps per SM with the L1 data pipe ~70% and the issue slots ~55% busy; HBM floor 0.24 ms.
 //
-// Precision: div u is the one sum whose terms (the velocity gradients) cancel by orders of
-// magnitude, and it multiplies rho, H and eta, so its line sums and fold run in FP64 (45 FP64
-// mul-adds of the ~450 packed ones).  The mass, energy and entropy residuals are then several
-// times closer to FP64 than with FP32 sums on affine deviations, which needed a second prologue
-// barrier and three fields more.
+// Precision.  div u cancels by orders of magnitude and multiplies rho, H and eta, so its line sums and
+// fold run in FP64.  The viscous terms differentiate twice, so an error in a gradient is raised by the
+// ratio of the flux to its divergence, ~n for n elements across a wave: the velocity gradients are those
+// FP64 line sums, rounded once, and T, like p, is held as the deviation from an affine reference (what is
+// left is second order in the element size).  With both from constant references in FP32 the launch took
+// 0.801 ms and the assembled viscous and heat terms were 2 to 3.5 times further from FP64 (shear, 48
+// elements, 5% jitter: 1.4e-5 against 4.0e-6; heat flux 3.4e-6 against 1.1e-6).
 #include "sod_internal.cuh"
 #include "sod_step_kernels.cuh"
 #include <cmath>
@@ -51,9 +53,9 @@ constexpr int NA = 4;    // nodal slots (field pairs)
 constexpr int NU = 3;    // FP64 velocity slots
 constexpr int NP2 = 9;   // pass-2 slots
 constexpr int NSLOT = NA + NU + NP2;
-// doubles per element ahead of the slots: rho, u, h, k, T of node 0; p of the nodes (0,0,0), (3,0,0),
-// (0,3,0), (0,0,3); log p and log rho of node 0; then FP32 references (8 floats) and the slopes of p (3)
-constexpr int R_P = 7, R_LOG = R_P + 4, R_F32 = R_LOG + 3, NREF = R_F32 + 6;
+// doubles per element ahead of the slots: rho, u, h, k of node 0; (p, T) of the nodes (0,0,0), (3,0,0),
+// (0,3,0), (0,0,3); log p and log rho of node 0; then FP32 references (7 floats) and the slopes of (p, T) (3)
+constexpr int R_P = 6, R_LOG = R_P + 8, R_F32 = R_LOG + 2, NREF = R_F32 + 4 + 4;
 constexpr int NDTAB = 32;  // doubles per CTA: D and D^T in FP32, then D; rows of 4
 
 __host__ __device__ constexpr size_t smem_bytes(int epb) {
@@ -124,6 +126,7 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
   const int ee = active ? e : a.nelem - 1;
   double* refs = refs_all + es * NREF;
   float* rf = reinterpret_cast<float*>(refs + R_F32);
+  float2* slopes = reinterpret_cast<float2*>(refs + R_F32 + 4);  // of (p, T) along xi, eta, zeta
   float2* buf = buf_all + (size_t)es * NSLOT * FSTRIDE;
   double* ud = reinterpret_cast<double*>(buf + NA * FSTRIDE);
   float2* p2 = buf + (NA + NU) * FSTRIDE;
@@ -160,12 +163,13 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
   // element references: FP64 values of local node 0, and their FP32 copies
   if (d == 0) {
     refs[0] = rho; refs[1] = uv[0]; refs[2] = uv[1]; refs[3] = uv[2];
-    refs[4] = h; refs[5] = kk; refs[6] = T;
+    refs[4] = h; refs[5] = kk;
     rf[0] = (float)rho; rf[1] = (float)uv[0]; rf[2] = (float)uv[1]; rf[3] = (float)uv[2];
-    rf[4] = (float)(h + kk); rf[5] = (float)irho; rf[6] = (float)T;
-    rf[7] = 1.0f / (float)p;
+    rf[4] = (float)(h + kk); rf[5] = (float)irho;
+    rf[6] = 1.0f / (float)p;
   }
-  if (d == 0 || d == 3 || d == 12 || d == 48) refs[R_P + (d == 0 ? 0 : (d == 3 ? 1 : (d == 12 ? 2 : 3)))] = p;
+  if (d == 0 || d == 3 || d == 12 || d == 48)
+    *reinterpret_cast<double2*>(refs + R_P + (d == 0 ? 0 : (d == 3 ? 2 : (d == 12 ? 4 : 6)))) = make_double2(p, T);
 #pragma unroll
   for (int c = 0; c < 3; ++c) ud[c * FSTRIDE + s_me] = uv[c];
   __syncthreads();
@@ -173,22 +177,31 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
   if ((lt & ~1) == 32) refs[R_LOG + (lt & 1)] = log((lt & 1) ? refs[0] : refs[R_P]);
   // deviations from node 0; L - L_r by log1p of small ratios
   const float drho = (float)(rho - refs[0]);
-  const double p0 = refs[R_P];
-  const float dL = log1pf((float)(p - p0) * rf[7]) - a.prm.gamma_f * log1pf(drho * rf[5]);
+  const double p0 = refs[R_P], T0 = refs[R_P + 1];
+  const float dL = log1pf((float)(p - p0) * rf[6]) - a.prm.gamma_f * log1pf(drho * rf[5]);
   float2 v0, v1, v2, v3;   // own slots
   {
     constexpr double kX = 0.44721359549995793928;  // interior GLL nodes of p = 3: +-sqrt(1/5)
     auto xh = [&](int t) {  // (xi_t + 1)/2
       return t == 0 ? 0.0 : (t == 1 ? 0.5 * (1.0 - kX) : (t == 2 ? 0.5 * (1.0 + kX) : 1.0));
     };
-    const double cx = refs[R_P + 1] - p0, cy = refs[R_P + 2] - p0, cz = refs[R_P + 3] - p0;
-    // p = p_0 + sum_d a_d (xi_d + 1) + p', a_d from the three corner nodes: D differentiates linear
-    // functions exactly, so D p = D p' + a
-    if (d < 3) rf[8 + d] = 0.5f * (float)(d == 0 ? cx : (d == 1 ? cy : cz));
+    // f = f_0 + sum_d a_d (xi_d + 1) + f' for f = p, T, a_d from the three corner nodes: D differentiates
+    // linear functions exactly, so D f = D f' + a
+    auto corner = [&](int t) {
+      const double2 c = *reinterpret_cast<const double2*>(refs + R_P + 2 * (t + 1));
+      return make_double2(c.x - p0, c.y - T0);
+    };
+    const double2 cx = corner(0), cy = corner(1), cz = corner(2);
+    if (d < 3) {
+      const double2 c = d == 0 ? cx : (d == 1 ? cy : cz);
+      slopes[d] = make_float2(0.5f * (float)c.x, 0.5f * (float)c.y);
+    }
+    const double wx = xh(i), wy = xh(j), wz = xh(k);
     v0 = make_float2((float)(uv[0] - refs[1]), (float)(uv[1] - refs[2]));
     v1 = make_float2((float)(uv[2] - refs[3]), (float)((h - refs[4]) + (kk - refs[5])));  // total enthalpy H = h + k
     v2 = make_float2(drho, (rf[0] + drho) * dL);
-    v3 = make_float2((float)((p - p0) - (cx * xh(i) + cy * xh(j) + cz * xh(k))), (float)(T - refs[6]));
+    v3 = make_float2((float)((p - p0) - (cx.x * wx + cy.x * wy + cz.x * wz)),
+                     (float)((T - T0) - (cx.y * wx + cy.y * wy + cz.y * wz)));
     buf[0 * FSTRIDE + s_me] = v0;
     buf[1 * FSTRIDE + s_me] = v1;
     buf[2 * FSTRIDE + s_me] = v2;
@@ -197,7 +210,7 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
   // full node values in FP32: reference + deviation
   const float uR[3] = {rf[1] + v0.x, rf[2] + v0.y, rf[3] + v1.x};
   const float HR = rf[4] + v1.y, rhoR = rf[0] + v2.x;
-  const float Tf = rf[6] + v3.y;
+  const float Tf = (float)T;
   const float muf = mufac * (float)kC1 * (Tf * sqrtf(Tf)) / (Tf + (float)kS);
   __syncthreads();
 
@@ -216,12 +229,14 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
     const int x = dir == 0 ? i : (dir == 1 ? j : k);
     float2 w[4];
     load_row(dtab, x, w);
-    float2 g0, g1, g2, g3;
+    float2 g2, g3;
+    float2 lu01;  // line sums of u, from FP64
+    float lu2;
     auto point = [&](int m, float2 p0, float2 p1, float2 p2_, float2 p3) {
       if (m == 0) {
-        g0 = MUL2(w[0], p0); g1 = MUL2(w[0], p1); g2 = MUL2(w[0], p2_); g3 = MUL2(w[0], p3);
+        g2 = MUL2(w[0], p2_); g3 = MUL2(w[0], p3);
       } else {
-        g0 = FMA2(w[m], p0, g0); g1 = FMA2(w[m], p1, g1); g2 = FMA2(w[m], p2_, g2); g3 = FMA2(w[m], p3, g3);
+        g2 = FMA2(w[m], p2_, g2); g3 = FMA2(w[m], p3, g3);
       }
       // differences to the own point
       const float2 d0 = ADD2(p0, make_float2(-v0.x, -v0.y)), d1 = ADD2(p1, make_float2(-v1.x, -v1.y)),
@@ -256,7 +271,9 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
 #pragma unroll
       for (int c = 0; c < 3; ++c, fu += FSTRIDE) {
         const double2 fa = *reinterpret_cast<const double2*>(fu), fb = *reinterpret_cast<const double2*>(fu + 2);
-        divU64 += (double)hc[c] * ((wa.x * fa.x + wa.y * fa.y) + (wb.x * fb.x + wb.y * fb.y));
+        const double l = (wa.x * fa.x + wa.y * fa.y) + (wb.x * fb.x + wb.y * fb.y);
+        divU64 += (double)hc[c] * l;
+        (c == 0 ? lu01.x : (c == 1 ? lu01.y : lu2)) = (float)l;
       }
     } else {
       const float2* f = buf + (dir == 1 ? sidx(i, 0, k) : sidx(i, j, 0));
@@ -267,16 +284,19 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
       const double2 wa = *reinterpret_cast<const double2*>(dtab64 + 4 * x),
                   wb = *reinterpret_cast<const double2*>(dtab64 + 4 * x + 2);
 #pragma unroll
-      for (int c = 0; c < 3; ++c, fu += FSTRIDE)
-        divU64 += (double)hc[c] * ((wa.x * fu[0] + wa.y * fu[st]) + (wb.x * fu[2 * st] + wb.y * fu[3 * st]));
+      for (int c = 0; c < 3; ++c, fu += FSTRIDE) {
+        const double l = (wa.x * fu[0] + wa.y * fu[st]) + (wb.x * fu[2 * st] + wb.y * fu[3 * st]);
+        divU64 += (double)hc[c] * l;
+        (c == 0 ? lu01.x : (c == 1 ? lu01.y : lu2)) = (float)l;
+      }
     }
-    g3.x += rf[8 + dir];  // the affine part of p
+    g3 = ADD2(g3, slopes[dir]);  // the affine parts of p and T
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       if (dir == 0) {
-        gU01[r] = MUL2(F2(hc[r]), g0); gU2[r] = hc[r] * g1.x; gRho[r] = hc[r] * g2.x; gT[r] = hc[r] * g3.y;
+        gU01[r] = MUL2(F2(hc[r]), lu01); gU2[r] = hc[r] * lu2; gRho[r] = hc[r] * g2.x; gT[r] = hc[r] * g3.y;
       } else {
-        gU01[r] = FMA2(F2(hc[r]), g0, gU01[r]); gU2[r] = fmaf(hc[r], g1.x, gU2[r]);
+        gU01[r] = FMA2(F2(hc[r]), lu01, gU01[r]); gU2[r] = fmaf(hc[r], lu2, gU2[r]);
         gRho[r] = fmaf(hc[r], g2.x, gRho[r]); gT[r] = fmaf(hc[r], g3.y, gT[r]);
       }
     }
