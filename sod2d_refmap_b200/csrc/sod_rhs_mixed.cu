@@ -28,7 +28,7 @@
 // ^ marks contravariant fluxes.  Every field is held as its deviation from an element reference
 // (node 0, in FP64, before the FP32 cast); p and T from one that is affine in xi.
 //
-// Measured at 64^3 (262,144 elements, one launch): 0.822 ms, 1.254 ms with the 12 gradient fields
+// Measured at 64^3 (262,144 elements, one launch): 0.836 ms, 1.254 ms with the 12 gradient fields
 // and 25 staged-factor products of the quartets formed one by one.  Bounded by latency at 20
 // resident warps per SM with the L1 data pipe ~70% and the issue slots ~55% busy; HBM floor 0.24 ms.
 //
@@ -39,6 +39,11 @@
 // left is second order in the element size).  With both from constant references in FP32 the launch took
 // 0.801 ms and the assembled viscous and heat terms were 2 to 3.5 times further from FP64 (shear, 48
 // elements, 5% jitter: 1.4e-5 against 4.0e-6; heat flux 3.4e-6 against 1.1e-6).
+// The momentum's sums are u . grad u: where it cancels between the three directions (a shear), the
+// rounding of each term V^ r^ du counts against a small result.  So V_x rho_x times the precise line sum
+// is split off and only the rest, second order in the element size, is summed point by point (14 us of
+// the launch): error of a shear's momentum 6e-9 of rho u du/dy where the unsplit sums had 6.2e-8, and in a
+// channel, where transport and viscous terms balance, 2.1e-7 of the residual against 2.3e-7 (24^3).
 #include "sod_internal.cuh"
 #include "sod_step_kernels.cuh"
 #include <cmath>
@@ -226,6 +231,7 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
     const float hc[3] = {H[dir], H[3 + dir], H[6 + dir]};
     const float hh[3] = {0.5f * hc[0], 0.5f * hc[1], 0.5f * hc[2]};
     const float Vx = fmaf(hc[2], uR[2], fmaf(hc[1], uR[1], hc[0] * uR[0]));
+    const float Vh = 0.5f * Vx;
     const int x = dir == 0 ? i : (dir == 1 ? j : k);
     float2 w[4];
     load_row(dtab, x, w);
@@ -241,15 +247,19 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
       // differences to the own point
       const float2 d0 = ADD2(p0, make_float2(-v0.x, -v0.y)), d1 = ADD2(p1, make_float2(-v1.x, -v1.y)),
                    d2 = ADD2(p2_, make_float2(-v2.x, -v2.y));
-      const float wV = w[m].x * fmaf(hh[2], d1.x, fmaf(hh[1], d0.y, fmaf(hh[0], d0.x, Vx)));  // D V^
-      const float2 s = F2(wV * fmaf(0.5f, d2.x, rhoR)), sv = F2(wV);                            // D V^ r^, D V^
+      // V^ = V_x + hV; s = D (V^ r^ - V_x rho_x) = D (hV r^ + V_x/2 drho), sv = D V^
+      const float hV = fmaf(hh[2], d1.x, fmaf(hh[1], d0.y, hh[0] * d0.x));
+      const float rh = fmaf(0.5f, d2.x, rhoR);
+      const float2 s = F2(w[m].x * fmaf(hV, rh, Vh * d2.x)), sv = F2(w[m].x * (Vx + hV));
       sum0 = FMA2(s, d0, sum0);
       sum2 = FMA2(sv, d2, sum2);
       if constexpr (TOTH) {
+        const float dG = fmaf(rhoR + d2.x, d1.y, HR * d2.x);  // rho_m dH + H drho
         sum1.x = fmaf(s.x, d1.x, sum1.x);
-        sum1.y = fmaf(wV, fmaf(rhoR + d2.x, d1.y, HR * d2.x), sum1.y);  // dG = rho_m dH + H drho
+        sum1.y = fmaf(sv.x, dG, sum1.y);
       } else {
-        sum1 = FMA2(s, d1, sum1);
+        sum1.x = fmaf(s.x, d1.x, sum1.x);
+        sum1.y = fmaf(sv.x * rh, d1.y, sum1.y);
       }
     };
     const double* fu = ud + (dir == 0 ? sidx(0, j, k) : (dir == 1 ? sidx(i, 0, k) : sidx(i, j, 0)));
@@ -291,6 +301,10 @@ __device__ __forceinline__ void rhs_mixed2_tile(const RhsArgs& a, int tile, unsi
       }
     }
     g3 = ADD2(g3, slopes[dir]);  // the affine parts of p and T
+    // momentum: the part of s taken out above, times the whole line sum
+    const float Wx = Vx * rhoR;
+    sum0 = FMA2(F2(Wx), lu01, sum0);
+    sum1.x = fmaf(Wx, lu2, sum1.x);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       if (dir == 0) {

@@ -1,12 +1,15 @@
-"""The viscous and heat-flux terms of the mixed right-hand side by themselves: states whose convective
-residual is far below the viscous one, against the FP64 path (1e-12 of the oracle).
+"""The viscous, heat-flux and momentum transport terms of the mixed right-hand side by themselves, against
+the FP64 path (1e-12 of the oracle): on the whole residual of a vortex the other terms hide them.
 
-Bound: a second derivative assembled from FP32 fluxes.  Each flux carries about ten roundings (gradient,
+Bound of the viscous and heat terms: a second derivative assembled from FP32 fluxes.  Each flux carries about ten roundings (gradient,
 metric, viscosity, gpvol, weak-divergence weights and sums) of 0.3 * 2^-24 rms that add like a random walk;
 the weak divergence (row norm 5.3 of D, 2/h = n/pi) raises them against the result, a factor k of the
 wave number smaller.  A 5% jitter of the nodes and unequal rows of D: half as much again.  Gradients of
 deviations that keep their linear part in FP32 exceed it: those lose the ratio of a field's variation over
-the element to its curvature."""
+the element to its curvature.
+
+Bound of the momentum transport of a shear (whose three directions cancel): one rounding, 0.3 * 2^-24 rms,
+of each direction's product at the full scale rho u du/dy."""
 import math
 
 import numpy as np
@@ -63,3 +66,14 @@ def test_heat_flux_at_rest(mods, n):
     got, ref = residuals(mods, n, lambda x, y, z: prm.p0 / (prm.Rgas * (300.0 + 5.0 * np.cos(3.0 * y))),
                          lambda x, y, z: np.zeros((x.size, 3)), lambda x, y, z: 0 * x + prm.p0, 1e4 * prm.mu_factor, 0.0)
     assert rel_l2(got["Rener"], ref["Rener"]) < bound(n, 3.0)
+
+
+@pytest.mark.parametrize("n", [8, 21, 32])
+def test_momentum_transport_of_a_shear(mods, n):
+    prm = mods[1].TGVParams()
+    rho = prm.p0 / (prm.Rgas * prm.T0)
+    got, ref = residuals(mods, n, lambda x, y, z: 0 * x + rho, lambda x, y, z: np.stack([np.sin(y), 0 * y, 0 * y], axis=1),
+                         lambda x, y, z: 0 * x + prm.p0, 0.0, 0.0)
+    d = got["Rmom"] - ref["Rmom"]
+    scale = rho / math.sqrt(8.0)  # rms of rho sin(y) cos(y)
+    assert np.linalg.norm(d) / math.sqrt(len(d)) < math.sqrt(3.0) * 0.3 * 2.0**-24 * scale
