@@ -77,3 +77,34 @@ def test_momentum_transport_of_a_shear(mods, n):
     d = got["Rmom"] - ref["Rmom"]
     scale = rho / math.sqrt(8.0)  # rms of rho sin(y) cos(y)
     assert np.linalg.norm(d) / math.sqrt(len(d)) < math.sqrt(3.0) * 0.3 * 2.0**-24 * scale
+
+
+def test_sgs_viscosity_product(mods):
+    """rho mu_sgs enters the stress as one FP64 product rounded once.  Two states with the same velocity,
+    pressure, and factors rho and mu_sgs / 4 of 1 and of a value just below the FP32 midpoint 1 + 2^-24.  The
+    products are 4 and about 4 (1 + 2^-23), which both round well; FP32 factors would round to 1 and 4 both
+    times, and the viscous momentum of the two states would not differ."""
+    torch, M, S = mods
+    m = M.periodic_box(6, jitter=0.0, seed=0)
+    prm = M.TGVParams(flag_les=1)
+    gm = S.Sod2dMesh(m, prm)
+    u = np.zeros((m.npoin, 3))
+    u[:, 0] = np.sin(m.coord[:, 1])
+    up = (1.0 + 2.0**-24) * (1.0 - 2.0**-28)
+    dt, R = 1e-3, []
+    for rho, mus in ((1.0, 4.0), (up, 4.0 * up)):
+        s = S.Sod2dState(m.npoin, m.nelem)
+        for t, a in ((s.u, u.T), (s.q, (rho * u).T), (s.E, prm.p0 / (prm.gamma_gas - 1.0) + 0.5 * rho * (u * u).sum(axis=1))):
+            t.copy_(torch.from_numpy(np.ascontiguousarray(a)))
+        s.rho.fill_(rho)
+        s.mu_factor.fill_(0.0)
+        s.mu_e.fill_(0.0)
+        s.mu_sgs.fill_(mus)
+        s.dt.fill_(dt)
+        stages = torch.empty(15 * m.npoin, dtype=torch.float64, device="cuda")
+        q = t2n(s.q)
+        gm.rk_4_main_record(s, stages, update_dt=False, precision=S.MIXED)
+        R.append((q - t2n(stages[m.npoin:4 * m.npoin].view(3, -1))) * 2.0 / dt)
+    # the other roundings are the same in both states or average out over the nodes
+    gain = np.vdot(R[1], R[0]) / np.vdot(R[0], R[0]) - 1.0
+    assert abs(gain - (up * up - 1.0)) < 2.0**-25, gain
