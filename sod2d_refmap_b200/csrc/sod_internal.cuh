@@ -92,6 +92,14 @@ struct DevParams {
 struct DMat {
   double d[NP1][NP1];
 };
+// Row sums of D: zero but for the rounding of its entries (as given by the caller), to double precision.
+inline void d_row_sums(const DMat& D, double (&s)[NP1]) {
+  for (int r = 0; r < NP1; ++r) {
+    long double t = 0.0L;
+    for (int c = 0; c < NP1; ++c) t += D.d[r][c];
+    s[r] = (double)t;
+  }
+}
 
 // Arguments of the fused element-RHS kernels.
 struct RhsArgs {

@@ -9,7 +9,7 @@
 // W(m) (of q), formed with the output point's metric, so nothing but the nodal fields is staged and
 // no product is differentiated by itself.  Lanes are ordered (i0 j0 i1 j1 k): a warp's xi and eta line
 // loads then cost one shared-memory wavefront each (see sod_rhs.cu).  20^3 elements:
-// convection 78 -> 25 us, diffusion 35 -> 27, scalar 22 -> 17, gather of 5 fields 15 -> 9.
+// convection 78 -> 27 us, diffusion 35 -> 27, scalar 22 -> 17, gather of 5 fields 15 -> 9.
 #include "sod_internal.cuh"
 #include <cmath>
 
@@ -41,6 +41,7 @@ struct RefArgs {
   const int32_t* econn;
   const double* geo;
   DMat D;
+  double Dsum[NP1];                             // row sums of D
   const double *u, *q, *rho, *pr, *E;          // convec / scalar
   const double *rho_n, *Tem, *mu_fluid;         // diffusion
   const double *mue, *musgs;                    // internal layout [e][64]
@@ -52,13 +53,23 @@ struct RefArgs {
 // whose energy residual is 0.5 (div((E + p) u) + (E + p) div u + u . grad(E + p)) with E the
 // total energy; mass and momentum are the same in both.  Both energy quartets (E and k = |u|^2/2, the
 // same form) are taken at once on H = E + k.
+//
+// u, q, rho and H enter the line sums by their differences to the own point, which are small on a resolved
+// field; the constant parts are whole sums (div u, div q, u.grad rho) times the own value, and D's row
+// sums, which are zero but for the rounding of D's entries.  The differences of H are formed from those of
+// E and k: the rounding of E + k itself would be differentiated.  Vortex at 8^3 against extended precision: mass
+// 3.1e-15, energy 3.4e-15, momentum less grad p 1.8e-16; with the quartets one by one 6.2e-15, 6.5e-15 and
+// 2.3e-16, with whole values in the sums 7.4e-15, 1.2e-14 and 3.3e-16 (and 24 us instead of 27 at 20^3).  On white
+// noise, where differences are no smaller than values, momentum 2.5e-16 (quartets 1.8e-16).
 template <bool TOTH>
 __global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefArgs a) {
-  __shared__ double f[9][FSTRIDE];  // rho, p, H (TOTH: p + E), u, q
-  __shared__ double Ds[16];
+  constexpr int F_K = TOTH ? 8 : 9;         // k, after
+  __shared__ double f[F_K + 1][FSTRIDE];   // rho, p, E (TOTH: p + E), u, q
+  __shared__ double Ds[16], Dsum[NP1];
   const int e = blockIdx.x;
   const Point p = point_of(threadIdx.x);
   if (threadIdx.x < 16) Ds[threadIdx.x] = a.D.d[threadIdx.x >> 2][threadIdx.x & 3];
+  if (threadIdx.x < NP1) Dsum[threadIdx.x] = a.Dsum[threadIdx.x];
   const int n = a.econn[(int64_t)e * NN + p.d];
   const int64_t N = a.npoin;
   const double* G = a.geo + (int64_t)e * NGEO * NN;
@@ -70,15 +81,18 @@ __global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefAr
 #pragma unroll
   for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; q[c] = a.q[n + N * c]; }
   const double rho = a.rho[n], El = a.E[n], pr = a.pr[n];
-  const double Hx = TOTH ? pr + El : El + 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-  f[0][p.s] = rho; f[1][p.s] = pr; f[2][p.s] = Hx;
+  const double Ex = TOTH ? pr + El : El, kx = 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  const double Hx = TOTH ? Ex : Ex + kx;
+  f[0][p.s] = rho; f[1][p.s] = pr; f[2][p.s] = Ex;
+  if (!TOTH) f[F_K][p.s] = kx;
 #pragma unroll
   for (int c = 0; c < 3; ++c) { f[3 + c][p.s] = u[c]; f[6 + c][p.s] = q[c]; }
   __syncthreads();
   double divU = 0.0, divQ = 0.0, ugr = 0.0;      // div u, div q, u.grad rho
-  double A[3] = {0, 0, 0}, B[3] = {0, 0, 0};     // div(q_c u) + rho div(u_c u); q.grad u_c + u.grad q_c
+  double A[3] = {0, 0, 0};                       // div(q_c u) + rho div(u_c u) + q.grad u_c + u.grad q_c, of the differences
   double gP[3] = {0, 0, 0};
-  double Ea = 0.0, Er = 0.0, Eb = 0.0;           // div(rho H u) + rho div(H u) (TOTH: div(H u)) less H times (Er = div(rho u), ..); the advective rest
+  double Ea = 0.0, Er = 0.0;                     // div(rho H u) + rho div(H u) + q.grad H + u.grad(rho H) (TOTH: div(H u) + u.grad H) and div(rho u), likewise
+  double sV = 0.0, sW = 0.0;                     // D's row sums times V and W
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
     const double h0 = H[dir], h1 = H[3 + dir], h2 = H[6 + dir];
@@ -90,45 +104,53 @@ __global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefAr
       const double w = Ds[4 * p.row[dir] + m];
       const double u_[3] = {v[3 * FSTRIDE], v[4 * FSTRIDE], v[5 * FSTRIDE]};
       const double q_[3] = {v[6 * FSTRIDE], v[7 * FSTRIDE], v[8 * FSTRIDE]};
-      const double r_ = v[0], H_ = v[2 * FSTRIDE];
+      const double r_ = v[0];
       const double wV = w * (h0 * u_[0] + h1 * u_[1] + h2 * u_[2]);
-      lr += w * r_;
+      const double dr = r_ - rho;
+      lr += w * dr;
       lp += w * v[FSTRIDE];
-      // H by its difference to the own point: the constant part of div(rho H u) + rho div(H u) and of
-      // u.grad(rho H) is H times small sums, formed once below
-      const double dH = H_ - Hx;
+      double dH = v[2 * FSTRIDE] - Ex;
+      if (!TOTH) dH += v[F_K * FSTRIDE] - kx;
       lH += w * dH;
       if (TOTH) {
         Ea += wV * dH;
       } else {
         const double wVr = wV * r_;
-        Er += wVr;
+        Er += wV * dr;
         Ea += (wVr + wV * rho) * dH;
         lrH += (w * r_) * dH;
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        A[c] += wV * (q_[c] + rho * u_[c]);
-        lu[c] += w * u_[c];
-        lq[c] += w * q_[c];
+        const double du = u_[c] - u[c], dq = q_[c] - q[c];
+        A[c] += wV * (dq + rho * du);
+        lu[c] += w * du;
+        lq[c] += w * dq;
       }
     }
+    sV += Vx * Dsum[p.row[dir]];
+    sW += Wx * Dsum[p.row[dir]];
     divU += h0 * lu[0] + h1 * lu[1] + h2 * lu[2];
     divQ += h0 * lq[0] + h1 * lq[1] + h2 * lq[2];
     ugr += Vx * lr;
     gP[0] += h0 * lp;
     gP[1] += h1 * lp;
     gP[2] += h2 * lp;
-    Eb += TOTH ? Vx * lH : Wx * lH + Vx * lrH;
+    Ea += TOTH ? Vx * lH : Wx * lH + Vx * lrH;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) B[c] += Wx * lu[c] + Vx * lq[c];
+    for (int c = 0; c < 3; ++c) A[c] += Wx * lu[c] + Vx * lq[c];
   }
+  // the constant parts
+  divU += sV;
+  divQ += sW;
+  ugr += rho * sV;
   const double Rm = 0.5 * (divQ + rho * divU + ugr);
-  const double Re = TOTH ? 0.5 * (Ea + 2.0 * Hx * divU + Eb)
-                         : 0.25 * (Ea + Eb + Hx * (Er + divQ + 2.0 * (rho * divU + ugr)));
+  const double Re = TOTH ? 0.5 * (Ea + Hx * (2.0 * divU + sV))
+                         : 0.25 * (Ea + Hx * (Er + divQ + 3.0 * rho * divU + 2.0 * ugr + sW));
+  const double cu = divQ + rho * divU + ugr + sW, cq = 2.0 * divU + sV;
   double Rmo[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) Rmo[c] = 0.25 * (A[c] + u[c] * divQ + q[c] * divU + B[c] + u[c] * ugr) + gP[c];
+  for (int c = 0; c < 3; ++c) Rmo[c] = 0.25 * (A[c] + u[c] * cu + q[c] * cq) + gP[c];
   store_res6<double>(a.rel, (size_t)e * NN + p.d, gpv * Rm, gpv * Rmo[0], gpv * Rmo[1], gpv * Rmo[2], gpv * Re, 0.0);
 }
 
@@ -397,6 +419,7 @@ static RefArgs ref_args(SodMesh* m) {
   a.econn = m->econn;
   a.geo = m->geo64;
   a.D = m->D;
+  d_row_sums(m->D, a.Dsum);
   a.rel = (double*)m->buf.rel;
   a.c_rho = m->prm.c_rho;
   a.c_ener = m->prm.c_ener;
