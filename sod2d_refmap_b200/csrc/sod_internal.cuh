@@ -116,6 +116,7 @@ struct RhsArgs {
   const double* __restrict__ mu_factor;  // per node
   void* rel;                       // R [(e*64 + d)*6 + f]
   DMat D;
+  double Dsum[NP1];                // row sums of D (FP64 kernels)
   float Df[NP1][NP1];              // D in FP32 (mixed kernels)
   DevParams prm;
 };

@@ -22,11 +22,14 @@
 //   (E+p)     G div u + sum_dir sum_m D[x][m] V^ dG          G = rho H, flag_total_enthalpy
 // (the energy is linear in (h, k) and every h term has a k twin, so both quartets are evaluated on
 // H).  These are the reference's sums with the products expanded around the output point, where
-// the constant parts vanish: 17 FP64 operations per line point instead of ~36, and none of the
-// derivatives of q, H, rho H, eta and their products.  Against the same formulas in 64 bits in
-// another order: 1.4e-13 (mass), 1.7e-12 (momentum) at 21^3, as the quartets formed one by one.
-// Measured at 64^3, one launch: 0.986 ms, 1.780 ms before; bounded by latency at 16 resident warps
-// with the FP64 pipe and the shared-memory pipe about equally loaded (~700 cycles each per element).
+// the constant parts vanish but for the row sums of D (its rounding), which are counted: 19 FP64 operations
+// per line point instead of ~36, and none of the derivatives of q, H, rho H, eta and their products.
+// u and rho enter the line sums as differences too, and u = q / rho is rounded once, since div u differentiates
+// that rounding.  Against extended precision, vortex at 8^3: mass 8.0e-15, energy 2.3e-14, entropy 2.0e-14;
+// quartets one by one 8.5e-15, 2.8e-14, 2.1e-14; with whole values of u in the sums, q * (1 / rho) and no
+// row sums 1.6e-14, 3.3e-14, 2.5e-14 (and 0.993 ms in what follows).
+// Measured at 64^3, one launch: 1.03 ms, 1.84 ms with the quartets one by one; bounded by latency at 16
+// resident warps with the FP64 pipe and the shared-memory pipe about equally loaded (~700 cycles each per element).
 //
 // This is the FP64 parity path.  The mixed path (FP32 element arithmetic on deviation fields) is
 // k_rhs_mixed2 in sod_rhs_mixed.cu.
@@ -51,7 +54,7 @@ __device__ __forceinline__ R divT(const R* fx, const R* fy, const R* fz, int i, 
 
 constexpr int NBUF = 8;  // rho, u0, u1, u2, H, eta, p, T
 constexpr int NP2 = 18;  // 6 contravariant fluxes x 3 directions
-constexpr int NDTAB = 32;  // per CTA: D rows, then D^T rows
+constexpr int NDTAB = 36;  // per CTA: D rows, then D^T rows, then D's row sums
 
 template <typename R>
 constexpr size_t rhs_smem_bytes(int epb) {
@@ -96,10 +99,17 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
   if (tid < 32) {
     const int r = (tid >> 2) & 3, c = tid & 3;
     dtab[tid] = tid < 16 ? a.D.d[r][c] : a.D.d[c][r];
+    if (tid < NP1) dtab[32 + tid] = a.Dsum[tid];
   }
+  const double* dsum = dtab + 32;
   // one reciprocal serves the divisions by rho; gamma/(gamma-1) and 1/Rgas come from the host
   const double irho = 1.0 / rho;
-  const double uv[3] = {qv[0] * irho, qv[1] * irho, qv[2] * irho};
+  double uv[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double t = qv[c] * irho;
+    uv[c] = t + (qv[c] - t * rho) * irho;  // rounded once: the rounding of u is differentiated in div u
+  }
   const double umag = uv[0] * uv[0] + uv[1] * uv[1] + uv[2] * uv[2];
   const double kk = 0.5 * umag;
   const double e_int = Et * irho - 0.5 * umag;
@@ -120,13 +130,14 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
 
   // ---- one pass over the line points
   double gradRho[3], gradU[3][3], gradT[3];
-  double Sm = 0.0, Sr = 0.0, Se = 0.0, Sn = 0.0;  // sum D V^ drho; D V^ r^; D V^ r^ dH (TOTH: D V^ dG); D V^ deta
-  double Su[3] = {0.0, 0.0, 0.0};                 // sum D V^ r^ u_c(m), + grad p below
+  double Sm = 0.0, Se = 0.0, Sn = 0.0;  // sum D V^ drho; D V^ r^ dH (TOTH: D V^ dG); D V^ deta
+  double Su[3] = {0.0, 0.0, 0.0};       // sum D V^ r^ du_c, + grad p below
+  double sV = 0.0;                      // D's row sums times V_x
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
     const double hc[3] = {H[dir], H[3 + dir], H[6 + dir]};
     const double hh[3] = {0.5 * hc[0], 0.5 * hc[1], 0.5 * hc[2]};
-    const double Vh = hh[0] * uv[0] + hh[1] * uv[1] + hh[2] * uv[2];  // V_x / 2
+    const double Vx = hc[0] * uv[0] + hc[1] * uv[1] + hc[2] * uv[2];
     const int x = dir == 0 ? i : (dir == 1 ? j : k);
     double w[4];
     {
@@ -141,26 +152,26 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
     for (int m = 0; m < 4; ++m) {
       const double* fm = f + m * stride[dir];
       const double r_ = fm[0];
-      const double u_[3] = {fm[FSTRIDE], fm[2 * FSTRIDE], fm[3 * FSTRIDE]};
+      const double du[3] = {fm[FSTRIDE] - uv[0], fm[2 * FSTRIDE] - uv[1], fm[3 * FSTRIDE] - uv[2]};
       const double H_ = fm[4 * FSTRIDE], n_ = fm[5 * FSTRIDE];
       gp += w[m] * fm[6 * FSTRIDE];
       gT += w[m] * fm[7 * FSTRIDE];
-      gr += w[m] * r_;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) gu[c] += w[m] * u_[c];
-      const double wV = w[m] * (Vh + (hh[0] * u_[0] + hh[1] * u_[1] + hh[2] * u_[2]));  // D V^
       const double dr = r_ - rho;
+      gr += w[m] * dr;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gu[c] += w[m] * du[c];
+      const double wV = w[m] * (Vx + (hh[0] * du[0] + hh[1] * du[1] + hh[2] * du[2]));  // D V^
       const double sr = wV * (rho + 0.5 * dr);
       Sm += wV * dr;
       Sn += wV * (n_ - eta);
-      Sr += sr;
       if constexpr (TOTH)
         Se += wV * (r_ * H_ - rho * Ht);
       else
         Se += sr * (H_ - Ht);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) Su[c] += sr * u_[c];
+      for (int c = 0; c < 3; ++c) Su[c] += sr * du[c];
     }
+    sV += Vx * dsum[x];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       if (dir == 0) {
@@ -177,13 +188,17 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
       Su[r] += hc[r] * gp;
     }
   }
+  // The row sums of D are its rounding: the reference's quartets hold 1.5, 1.5 and 1.75 times sV of the
+  // constant parts that the differences leave out (the diffusion's gradients none that counts).
   const double divU = gradU[0][0] + gradU[1][1] + gradU[2][2];
-  const double Rm = rho * divU + Sm;
-  const double Rn = eta * divU + Sn;
-  const double Re = TOTH ? rho * Ht * divU + Se : Ht * Rm + Se;
+  const double divS = divU + 1.5 * sV;
+  const double Rm = rho * divS + Sm;
+  const double Rn = eta * divS + Sn;
+  const double Rc = Rm + 0.25 * rho * sV;
+  const double Re = TOTH ? rho * Ht * divS + Se : Ht * Rc + Se;
   double Rmo[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) Rmo[c] = uv[c] * (Rm - Sr) + Su[c];
+  for (int c = 0; c < 3; ++c) Rmo[c] = uv[c] * Rc + Su[c];
 
   // ---- diffusion pass 1 (elem_diffu.f90:70-140): stresses and contravariant fluxes
   {
@@ -239,8 +254,9 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
   }
 }
 
-// Resident 64-thread element groups per SM the register budget must allow: 8 (128 registers, no
-// spill) 0.986 ms at 64^3, 6 (154 registers) 1.087 ms; 10 (96 registers) would spill 244 bytes.
+// Resident 64-thread element groups per SM the register budget must allow: 8 (128 registers; total
+// enthalpy spills 4 bytes).  Measured at 64^3 with whole values of u: 8 0.986 ms, 6 (154 registers) 1.087 ms;
+// 10 (96 registers) would have spilled 244 bytes.
 #ifndef SOD_KR64_MIN_CTAS
 #define SOD_KR64_MIN_CTAS 8
 #endif
@@ -428,6 +444,7 @@ static RhsArgs make_rhs_args(SodMesh* m, bool mixed, const double* rho, const do
   a.mu_factor = mu_factor;
   a.rel = m->buf.rel;
   a.D = m->D;
+  d_row_sums(m->D, a.Dsum);
   for (int r = 0; r < NP1; ++r)
     for (int c = 0; c < NP1; ++c) a.Df[r][c] = (float)m->D.d[r][c];
   a.prm = m->prm;

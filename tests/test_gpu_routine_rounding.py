@@ -1,4 +1,4 @@
-"""Rounding of full_convec_ijk on smooth fields, against the reference's quartets (elem_convec.f90:412-432)
+"""Rounding of the FP64 convection on smooth fields, against the reference's quartets (elem_convec.f90:412-432)
 in extended precision on the same metric and inputs.
 
 Bound: with the fields entering the line sums by their differences to the own point, a sum's terms are the
@@ -8,6 +8,8 @@ with the metric's.  Whole values in the sums round at |f| / h instead of |grad f
 refinement."""
 import numpy as np
 import pytest
+
+from _util import t2n
 
 pytestmark = pytest.mark.gpu
 LD = np.longdouble
@@ -38,6 +40,21 @@ def quartets(D, H, gpv, u, q, rho, pr, E):
     return [gpv * r for r in (Rm, *Rmo, Re)]
 
 
+def geometry(m, gm):
+    """Element nodes in i + 4j + 16k order, D, the library's own He and gpvol, and Ml."""
+    T, geo = m.tables, gm.geometry()
+    order = np.argsort(T.nat_ijk[:, 0] + 4 * T.nat_ijk[:, 1] + 16 * T.nat_ijk[:, 2])
+    f = lambda a: a[order].T.reshape(-1, 4, 4, 4).astype(LD)
+    H = [[f(geo["He"][c, d]) for d in range(3)] for c in range(3)]
+    return m.connec[:, order], np.asarray(T.D).astype(LD), H, f(geo["gpvol"][0]), geo["Ml"]
+
+
+def assemble(m, conn, r):
+    out = np.zeros(m.npoin, dtype=LD)
+    np.add.at(out, conn.ravel(), r.ravel())
+    return out
+
+
 @pytest.mark.parametrize("n", [8, 12])
 @pytest.mark.parametrize("flow", ["vortex", "shear"])
 def test_convection_of_smooth_fields(n, flow):
@@ -47,9 +64,8 @@ def test_convection_of_smooth_fields(n, flow):
     from sod2d_refmap_b200 import build, mesh as M, solver as S
     build.build()
     m, prm = M.periodic_box(n, jitter=0.05, seed=11), M.TGVParams()
-    gm, T = S.Sod2dMesh(m, prm), m.tables
-    order = np.argsort(T.nat_ijk[:, 0] + 4 * T.nat_ijk[:, 1] + 16 * T.nat_ijk[:, 2])
-    conn, geo = m.connec[:, order], gm.geometry()
+    gm = S.Sod2dMesh(m, prm)
+    conn, D, H, gpv, Ml = geometry(m, gm)
     x, y, z = m.coord.T
     if flow == "vortex":
         u = np.stack([np.sin(x) * np.cos(y) * np.cos(z), -np.cos(x) * np.sin(y) * np.cos(z), 0 * x])
@@ -61,12 +77,38 @@ def test_convection_of_smooth_fields(n, flow):
     Rm, Rmo, Re = gm.full_convec_ijk(dev(u), dev(q), dev(rho), dev(pr), dev(E))
     got = [Rm.cpu().numpy(), *Rmo.cpu().numpy(), Re.cpu().numpy()]
     el = lambda a: a[conn].reshape(-1, 4, 4, 4).astype(LD)
-    H = [[geo["He"][c, d][order].T.reshape(-1, 4, 4, 4).astype(LD) for d in range(3)] for c in range(3)]
-    gpv = geo["gpvol"][0][order].T.reshape(-1, 4, 4, 4).astype(LD)
-    ref = quartets(np.asarray(T.D).astype(LD), H, gpv, [el(a) for a in u], [el(a) for a in q], el(rho), el(pr), el(E))
+    ref = quartets(D, H, gpv, [el(a) for a in u], [el(a) for a in q], el(rho), el(pr), el(E))
     scale = 1.0 / np.sqrt(2.0)  # rms of |grad u|
     for i, f in ((0, 1.0), (1, 0.5), (2, 0.5), (4, 180.0)):
-        r = np.zeros(m.npoin, dtype=LD)
-        np.add.at(r, conn.ravel(), ref[i].ravel())
-        err = np.sqrt(np.mean(((got[i] - r).astype(float) / geo["Ml"])**2))
+        err = np.sqrt(np.mean(((got[i] - assemble(m, conn, ref[i])).astype(float) / Ml)**2))
         assert err < 2.0 * 2.0**-53 * f * scale, (i, err / (2.0**-53 * f * scale))
+
+
+@pytest.mark.parametrize("n", [8, 12])
+def test_fused_mass_residual_of_a_shear(n):
+    """The FP64 stage residual: div u of the velocity q / rho that the kernel forms itself, on a flow without
+    divergence.  The same bound for the mass residual (one divergence)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from sod2d_refmap_b200 import build, mesh as M, solver as S
+    build.build()
+    m, prm = M.periodic_box(n, jitter=0.05, seed=11), M.TGVParams()
+    gm, s = S.Sod2dMesh(m, prm), S.Sod2dState(m.npoin, m.nelem)
+    rho = prm.p0 / (prm.Rgas * prm.T0)
+    u = np.sin(m.coord[:, 1])
+    q = rho * u
+    s.rho.fill_(rho)
+    s.q.zero_()
+    s.q[0].copy_(torch.from_numpy(q))
+    s.E.copy_(torch.from_numpy(prm.p0 / (prm.gamma_gas - 1.0) + 0.5 * rho * u * u))
+    s.mu_factor.fill_(0.0)
+    s.mu_e.fill_(0.0)
+    got = t2n(gm.rhs(s, precision=S.FP64)["Rmass"])
+    conn, D, H, gpv, Ml = geometry(m, gm)
+    el = lambda a: a[conn].reshape(-1, 4, 4, 4).astype(LD)
+    Q = [el(q), el(0 * q), el(0 * q)]
+    R = LD(rho) + 0 * Q[0]
+    ref = assemble(m, conn, quartets(D, H, gpv, [c / R for c in Q], Q, R, 0 * R, 0 * R)[0])
+    err = np.sqrt(np.mean((got - (ref / Ml).astype(float))**2))
+    assert err < 2.0 * 2.0**-53 * rho / np.sqrt(2.0)
