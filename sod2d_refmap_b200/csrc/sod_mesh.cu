@@ -256,7 +256,7 @@ int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStr
 
 __global__ void k_inverse(int64_t n, const double* __restrict__ v, double* __restrict__ out) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) out[t] = v[t] != 0.0 ? 1.0 / v[t] : 0.0;
+  if (t < n) out[t] = 1.0 / v[t];
 }
 
 // Local node order of the library (natural d = i + 4j + 16k) from the reference's gmshAtoI/J/K
