@@ -190,6 +190,10 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
     k_fill<<<64, 256>>>(m->elem_member + eo, Ei, i);
     g_launches.fetch_add(5);
   }
+  if (int rc = mesh_init_node_data(m)) {
+    sod_batch_destroy(B);
+    return rc;
+  }
   cudaError_t err = cudaDeviceSynchronize();
   if (err != cudaSuccess) {
     set_error("sod_batch_create: %s", cudaGetErrorString(err));

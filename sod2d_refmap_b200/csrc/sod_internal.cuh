@@ -368,6 +368,8 @@ int mesh_from_device_ref(int nelem, int npoin, int base, const int32_t* connec, 
                          const int32_t* gI, const int32_t* gJ, const int32_t* gK, const double* wgp,
                          const double* helem_l, const double* helem, int npoin_w, const int32_t* lpoin_w,
                          const SodParams* params, cudaStream_t st, SodMesh** out);
+// scalars, counters and 1 / Ml of a mesh whose Ml is set (on the default stream; the caller waits)
+int mesh_init_node_data(SodMesh* m);
 // f32_copy (optional): FP32 copy of the internal array
 int mesh_ref_to_internal_elem(SodMesh* m, const double* ref_dev /*(nelem,64) F*/, double* int_dev,
                               cudaStream_t st, float* f32_copy = nullptr);

@@ -290,6 +290,28 @@ int mesh_set_local_tables(SodMesh* m, const int32_t* gI, const int32_t* gJ, cons
   return SOD_OK;
 }
 
+int mesh_init_scalars(SodMesh* m) {
+  StepBuffers& b = m->buf;
+  if (!b.scal) {
+    SOD_CUDA(cudaMalloc(&b.scal, sizeof(double) * 16));
+    SOD_CUDA(cudaMemset(b.scal, 0, sizeof(double) * 16));
+  }
+  if (!b.counters) {
+    SOD_CUDA(cudaMalloc(&b.counters, sizeof(unsigned int) * 16));
+    SOD_CUDA(cudaMemset(b.counters, 0, sizeof(unsigned int) * 16));
+  }
+  return SOD_OK;
+}
+// Formed with the mesh, not on the first call: a first call would pay an allocation, a launch and a wait.
+int mesh_init_node_data(SodMesh* m) {
+  const int64_t N = m->npoin;
+  if (int rc = mesh_init_scalars(m)) return rc;
+  SOD_CUDA(cudaMalloc(&m->buf.iml, sizeof(double) * N));
+  k_inverse<<<(unsigned)((N + 255) / 256), 256>>>(N, m->Ml, m->buf.iml);
+  SOD_CHECK_LAUNCH();
+  return SOD_OK;
+}
+
 int ensure_step_buffers(SodMesh* m, bool mixed) {
   if (int rc = init_kernel_attrs()) return rc;
   StepBuffers& b = m->buf;
@@ -299,21 +321,10 @@ int ensure_step_buffers(SodMesh* m, bool mixed) {
     SOD_CUDA(cudaMalloc(&b.rsum, sizeof(double) * 6 * N));
     b.red_cap = 4 * ((N + 127) / 128 + (E + 1) + 1024);
     SOD_CUDA(cudaMalloc(&b.red, sizeof(double) * b.red_cap));
-    SOD_CUDA(cudaMalloc(&b.scal, sizeof(double) * 16));
-    SOD_CUDA(cudaMemset(b.scal, 0, sizeof(double) * 16));
-    SOD_CUDA(cudaMalloc(&b.counters, sizeof(unsigned int) * 16));
-    SOD_CUDA(cudaMemset(b.counters, 0, sizeof(unsigned int) * 16));
     SOD_CUDA(cudaMalloc(&b.mu_fluid, sizeof(double) * N));
   }
-  bool filled = false;  // by kernels on the default stream, which the caller's stream may not wait for
-  if (!b.iml && m->Ml) {  // (a mesh view of the sod_*_ref entries has no lumped mass and no step)
-    double* v = nullptr;
-    SOD_CUDA(cudaMalloc(&v, sizeof(double) * N));
-    b.iml = v;
-    k_inverse<<<(unsigned)((N + 255) / 256), 256>>>(N, m->Ml, v);
-    SOD_CHECK_LAUNCH();
-    filled = true;
-  }
+  if (int rc = mesh_init_scalars(m)) return rc;  // a mesh view of the sod_*_ref entries; the others have them
+  bool filled = false;  // on the default stream, which the caller's stream may not wait for
   size_t need = (size_t)E * NRES * NN * sizeof(double);  // sized for FP64 (also holds FP32)
   if (b.rel_bytes < need) {
     if (b.rel) cudaFree(b.rel);
@@ -633,6 +644,7 @@ int sod_mesh_create(const SodMeshDesc* desc, const SodParams* params, SodMesh** 
     k_lumped_mass<<<(N + 255) / 256, 256>>>(N, m->n2e_ptr, m->n2e, m->geo64, m->Ml);
     g_launches.fetch_add(1);
   }
+  if (int rc = mesh_init_node_data(m)) return fail(rc);
   cudaError_t err = cudaDeviceSynchronize();
   if (err != cudaSuccess) {
     set_error("mesh create: %s", cudaGetErrorString(err));

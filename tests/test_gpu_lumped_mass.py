@@ -38,3 +38,22 @@ def test_zero_on_a_working_row_is_not_hidden(mods, precision):
     with pytest.raises(RuntimeError):
         gm.check_finite()
     assert not bool(torch.isfinite(s.rho[7]))
+
+
+def test_first_call_launches_no_more_than_the_second(mods):
+    """What depends on the mesh alone is formed with the handle: the FP64 right-hand side, its adjoint and a routine."""
+    torch, M, S = mods
+    from sod2d_refmap_b200 import _lib
+    m, prm = M.periodic_box(3, jitter=0.05, seed=1), M.TGVParams()
+    st = M.taylor_green_state(m, prm)
+    calls = (lambda g, s: g.rhs(s, precision=S.FP64),
+             lambda g, s: g.rhs_vjp(s.rho, s.q, s.E, s.mu_e, s.mu_factor, s.rho, s.q, s.E),
+             lambda g, s: g.full_convec_ijk(s.u, s.q, s.rho, s.pr, s.E))
+    for call in calls:
+        gm = S.Sod2dMesh(m, prm)
+        s = S.Sod2dState.from_host(st, gm.nelem)
+        counts = [_lib.launch_count()]
+        for _ in range(2):
+            call(gm, s)
+            counts.append(_lib.launch_count())
+        assert counts[1] - counts[0] == counts[2] - counts[1]
