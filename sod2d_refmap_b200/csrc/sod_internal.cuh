@@ -187,7 +187,6 @@ struct StepBuffers {
   double* scal = nullptr;    // device scalars: [0] eta mean, [1] eta norm, [2] dt, [3] ...
   unsigned int* counters = nullptr;  // last-block-done counters
   double* iml = nullptr;             // 1 / Ml per node (not read on rows without elements)
-  double* mu_fluid = nullptr;        // stage Sutherland viscosity scratch (unused by fused path)
 };
 
 struct GraphEntry {

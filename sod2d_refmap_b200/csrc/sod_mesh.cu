@@ -321,7 +321,6 @@ int ensure_step_buffers(SodMesh* m, bool mixed) {
     SOD_CUDA(cudaMalloc(&b.rsum, sizeof(double) * 6 * N));
     b.red_cap = 4 * ((N + 127) / 128 + (E + 1) + 1024);
     SOD_CUDA(cudaMalloc(&b.red, sizeof(double) * b.red_cap));
-    SOD_CUDA(cudaMalloc(&b.mu_fluid, sizeof(double) * N));
   }
   if (int rc = mesh_init_scalars(m)) return rc;  // a mesh view of the sod_*_ref entries; the others have them
   bool filled = false;  // on the default stream, which the caller's stream may not wait for
@@ -430,7 +429,7 @@ void sod_mesh_destroy(SodMesh* m) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   void* ptrs[] = {m->econn, m->geo64, m->geo32, m->Ml, m->helem, m->helem_l, m->jratio, m->n2e_ptr, m->n2e,
                   m->mue_int, m->mue32, m->a_of_d_dev, m->buf.ys, m->buf.rsum, m->buf.rel, m->buf.red,
-                  m->buf.scal, m->buf.counters, m->buf.mu_fluid, m->buf.iml, m->adj, m->musgs_int};
+                  m->buf.scal, m->buf.counters, m->buf.iml, m->adj, m->musgs_int};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (double* p : m->host_mirror) cudaFree(p);
