@@ -339,6 +339,7 @@ struct SodMesh {
   int32_t* member_node_off = nullptr;  // [nmember+1] contiguous node ranges
   double* member_scal = nullptr;    // [nmember][2] eta mean, eta norm
   double* member_dt_bits = nullptr; // [nmember] scratch for the per-member dt min
+  int nsm = 148;                    // SMs of the device (set with the mesh's node data)
   double* member_red = nullptr;     // [nmember][kEtaChunks][3] partial entropy sums
   unsigned int* member_done = nullptr;  // [nmember] chunks finished (zero between launches)
   double* musgs_int = nullptr;  // LES: internal-layout SGS viscosity (FP64), allocated on first use

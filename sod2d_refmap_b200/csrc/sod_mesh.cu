@@ -305,6 +305,9 @@ int mesh_init_scalars(SodMesh* m) {
 // Formed with the mesh, not on the first call: a first call would pay an allocation, a launch and a wait.
 int mesh_init_node_data(SodMesh* m) {
   const int64_t N = m->npoin;
+  int dev = 0;
+  SOD_CUDA(cudaGetDevice(&dev));
+  SOD_CUDA(cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, dev));
   if (int rc = mesh_init_scalars(m)) return rc;
   SOD_CUDA(cudaMalloc(&m->buf.iml, sizeof(double) * N));
   k_inverse<<<(unsigned)((N + 255) / 256), 256>>>(N, m->Ml, m->buf.iml);

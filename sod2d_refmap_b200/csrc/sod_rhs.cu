@@ -537,15 +537,15 @@ __global__ void __launch_bounds__(1024) k_eta_combine(int nblk, int nwork, int n
   }
 }
 
-// Stage 4 forms the entropy normalisation too.  While its blocks are all resident at once (one wave,
-// kOneWave), the last of them does it; beyond, every block would hold its SM slot for the fence and the
+// Stage 4 forms the entropy normalisation too.  While its blocks are all resident at once (one wave:
+// kGatherResident per SM), the last of them does it; beyond, every block would hold its SM slot for the fence and the
 // atomic (~1 us of a ~4 us block), so the block sums go to a launch of their own: 64^3, 27,648 blocks,
 // 458 -> 368 us mixed for 17 us more.
-constexpr int kOneWave = 148 * 4;
+constexpr int kGatherResident = 4;
 int launch_gather(SodMesh* m, bool mixed, int stage, GatherArgs& a, cudaStream_t st) {
   fill_gather_args(m, stage, a);
   const int nblk = (a.npoin + 255) / 256;
-  const bool apart = stage == 4 && !a.member_reduce && nblk > kOneWave;
+  const bool apart = stage == 4 && !a.member_reduce && nblk > kGatherResident * m->nsm;
   if (apart) a.counter = nullptr;
   if (int rc = mixed ? launch_gather_t<float>(stage, a, st) : launch_gather_t<double>(stage, a, st)) return rc;
   if (apart) {

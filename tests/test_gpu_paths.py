@@ -1,6 +1,7 @@
 """Branches of the kernels' launch rules at the sizes where they change: the Poisson node kernels in
 one trip and grid-stride, ensemble members beyond one chunk round of the entropy statistics, the
-shock sensor on both sides of its cap, and the per-routine kernels on unrelated u, q and E.
+stage-4 entropy sums within and beyond one wave of blocks, the shock sensor on both sides of its cap, and
+the per-routine kernels on unrelated u, q and E.
 
 Bounds: 1e-12 relative per field, the FP64 path's bound (each compares sums of the same terms in
 another order)."""
@@ -135,3 +136,20 @@ def test_routines_on_unrelated_fields(mods, oracle, n):
         for g, r in zip(got, ref):
             assert rel_l2(t2n(g), r) < TOL64
     assert rel_l2(t2n(gm.generic_scalar_convec_ijk(d(q), d(eta), d(u))), oracle.scalar_convec(om, q, eta, u)) < TOL64
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [17, 18])  # 519 and 616 blocks of the stage-4 gather: within and beyond one wave of 4 x 148
+def test_entropy_normalisation_around_one_wave(mods, n, precision):
+    """The step's mean and norm of the entropy (formed by the gather's last block, or by a launch of their
+    own) against smart_visc_spectral on the fields the step left, whose norm comes from another kernel."""
+    torch, M, S = mods
+    m, prm = M.periodic_box(n, jitter=0.05, seed=6), M.TGVParams()
+    gm = S.Sod2dMesh(m, prm)
+    s = S.Sod2dState.from_host(M.taylor_green_state(m, prm, 1e-2, seed=6), gm.nelem)
+    s.dt.fill_(1e-3)
+    gm.rk_4_main(s, S.FP64 if precision == "fp64" else S.MIXED)
+    ref = gm.smart_visc_spectral(s.Reta, s.rho, s.u, s.csound, s.Tem, s.eta)
+    spread = float((s.eta - s.eta.mean()).abs().max() / s.eta.abs().max())
+    # the norm is a difference of FP64 sums of N terms: N^(1/2) roundings of the mean against the spread
+    assert rel_l2(t2n(s.mu_e), t2n(ref)) < 4 * m.npoin**0.5 * 2.0**-53 / spread
