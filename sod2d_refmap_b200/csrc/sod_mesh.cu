@@ -241,12 +241,8 @@ int mesh_ref_to_internal_elem(SodMesh* m, const double* ref, double* out, cudaSt
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
-// One launch, except for steps with one-launch stages (sod_set_stage_launch), whose launch count callers
-// check: there the FP32 copy stays a launch of its own.
 int mesh_mue_in(SodMesh* m, const double* mu_e, bool mixed, cudaStream_t st) {
-  const bool apart = mixed && m->persist_ctas[1] > 0;
-  if (int rc = mesh_ref_to_internal_elem(m, mu_e, m->mue_int, st, mixed && !apart ? m->mue32 : nullptr)) return rc;
-  return apart ? launch_copy_f32(m->mue_int, m->mue32, (int64_t)m->nelem * NN, st) : SOD_OK;
+  return mesh_ref_to_internal_elem(m, mu_e, m->mue_int, st, mixed ? m->mue32 : nullptr);
 }
 int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStream_t st) {
   k_int2ref<<<(m->nelem + kTileE - 1) / kTileE, 256, 0, st>>>(m->nelem, m->a_of_d_dev, in, ref);

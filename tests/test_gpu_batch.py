@@ -152,8 +152,7 @@ def test_one_launch_stage_matches_two_launches(prec):
     n0 = _lib.launch_count()
     gm.rk_4_main(x, precision=p, update_dt=True)
     n1 = _lib.launch_count()
-    extra = 2 if prec == "MIXED" else 1              # the mu_e layout copies (and its FP32 copy)
-    assert n1 - n0 == 4 + 1 + extra, n1 - n0
+    assert n1 - n0 == 4 + 2, n1 - n0                 # four stages and a mu_e layout copy each way
     gm.rk_4_main(y, precision=p, update_dt=True)
     gm.rk4_steps(y, 1, precision=p)
     torch.cuda.synchronize()
