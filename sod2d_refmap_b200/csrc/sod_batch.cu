@@ -147,7 +147,6 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
   BALLOC(m->helem_l, sizeof(double) * E * NN);
   BALLOC(m->jratio, sizeof(double) * E);
   BALLOC(m->mue_int, sizeof(double) * E * NN);
-  BALLOC(m->a_of_d_dev, sizeof(int32_t) * NN);
   BALLOC(m->node_member, sizeof(int32_t) * N);
   BALLOC(m->elem_member, sizeof(int32_t) * E);
   BALLOC(m->member_node_off, sizeof(int32_t) * (nmesh + 1));
@@ -166,7 +165,6 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
     BALLOC(B->st.mu_e, sizeof(double) * E * NN);
   }
 #undef BALLOC
-  cudaMemcpy(m->a_of_d_dev, m0->a_of_d_dev, sizeof(int32_t) * NN, cudaMemcpyDeviceToDevice);
   cudaMemset(m->mue_int, 0, sizeof(double) * E * NN);
   cudaMemset(m->member_done, 0, sizeof(unsigned int) * nmesh);
   cudaMemset(B->st.mu_e, 0, sizeof(double) * E * NN);

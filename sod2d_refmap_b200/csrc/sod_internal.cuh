@@ -319,7 +319,7 @@ struct SodMesh {
   int32_t* n2e = nullptr;
   double* mue_int = nullptr;   // internal-layout entropy viscosity (FP64)
   float* mue32 = nullptr;      // FP32 copy
-  int32_t* a_of_d_dev = nullptr;  // perm table on device (64)
+  int32_t* a_of_d_dev = nullptr;  // perm_a_of_d on the device (mesh views of the sod_*_ref entries)
   sod::StepBuffers buf;
   std::unordered_map<uint64_t, sod::GraphEntry> graphs;
   int tuned_epb[2] = {0, 0};

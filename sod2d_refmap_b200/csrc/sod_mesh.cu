@@ -187,69 +187,74 @@ int launch_copy_f32(const double* src, float* dst, int64_t n, cudaStream_t st) {
   return SOD_OK;
 }
 
-// reference (nelem,64) F layout <-> internal [e*64+d]: a 32-element x 64-node tile goes through
-// shared memory, so that both sides move whole 256-byte rows (a thread per value read or wrote
-// 8 bytes of 64 different columns).  mue32 (optional): FP32 copy of the internal array, formed on the
-// way.  64^3, 134 MB each way: in 54 us with the FP32 copy (83 + 30 in two kernels before),
-// out 39 us (110 before).
-constexpr int kTileE = 32;
-__global__ void __launch_bounds__(256) k_ref2int(int nelem, const int32_t* __restrict__ a_of_d,
+// reference (nelem,64) F layout <-> internal [e*64+d]: a tile of 32 elements x 32 nodes goes through
+// shared memory, so that both sides move whole 256-byte rows (a thread per value read or wrote 8 bytes of
+// 64 different columns).  out32 (optional): FP32 copy of the internal array, formed on the way.  Tiles of all 64
+// nodes leave most of the chip idle on a small mesh, tiles of 16 take 25% longer on a large one.  In (with the
+// copy) / out, us: 4^3 1.8 / 1.7, 24^3 3.6 / 3.2, 64^3 (134 MB each way) 54 / 37; a thread per value
+// (copy apart) 3.6 / 1.8, 9.7 / 7.6, 113 / 112; tiles of 64 nodes 2.5 / 2.1, 3.6 / 3.5, 54 / 39.
+constexpr int kTileE = 32, kTileD = 32;
+struct NodePerm {
+  int a[NN];  // reference node of internal node d
+};
+__global__ void __launch_bounds__(256) k_ref2int(int nelem, const __grid_constant__ NodePerm perm,
                                                  const double* __restrict__ ref, double* __restrict__ out,
                                                  float* __restrict__ out32) {
-  __shared__ double tile[NN][kTileE + 1];  // [reference node a][element]
-  __shared__ int ad[NN];
-  const int e0 = blockIdx.x * kTileE, ne = min(kTileE, nelem - e0);
-  if (threadIdx.x < NN) ad[threadIdx.x] = a_of_d[threadIdx.x];
+  __shared__ double tile[kTileD][kTileE + 1];
+  const int e0 = blockIdx.x * kTileE, ne = min(kTileE, nelem - e0), d0 = blockIdx.y * kTileD;
 #pragma unroll
-  for (int q = 0; q < NN * kTileE / 256; ++q) {
-    const int t = q * 256 + threadIdx.x, le = t % kTileE, an = t / kTileE;
-    if (le < ne) tile[an][le] = ref[e0 + le + (int64_t)nelem * an];
+  for (int q = 0; q < kTileD * kTileE / 256; ++q) {
+    const int t = q * 256 + threadIdx.x, le = t % kTileE, d = t / kTileE;
+    if (le < ne) tile[d][le] = ref[e0 + le + (int64_t)nelem * perm.a[d0 + d]];
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < NN * kTileE / 256; ++q) {
-    const int t = q * 256 + threadIdx.x, le = t >> 6, d = t & 63;
+  for (int q = 0; q < kTileD * kTileE / 256; ++q) {
+    const int t = q * 256 + threadIdx.x, le = t / kTileD, d = t % kTileD;
     if (le < ne) {
-      const double v = tile[ad[d]][le];
-      out[(int64_t)e0 * NN + t] = v;
-      if (out32) out32[(int64_t)e0 * NN + t] = (float)v;
+      const double v = tile[d][le];
+      const int64_t o = (int64_t)(e0 + le) * NN + d0 + d;
+      out[o] = v;
+      if (out32) out32[o] = (float)v;
     }
   }
 }
-__global__ void __launch_bounds__(256) k_int2ref(int nelem, const int32_t* __restrict__ a_of_d,
+__global__ void __launch_bounds__(256) k_int2ref(int nelem, const __grid_constant__ NodePerm perm,
                                                  const double* __restrict__ in, double* __restrict__ ref) {
-  __shared__ double tile[NN][kTileE + 1];
-  __shared__ int ad[NN];
-  const int e0 = blockIdx.x * kTileE, ne = min(kTileE, nelem - e0);
-  if (threadIdx.x < NN) ad[threadIdx.x] = a_of_d[threadIdx.x];
-  __syncthreads();
+  __shared__ double tile[kTileD][kTileE + 1];
+  const int e0 = blockIdx.x * kTileE, ne = min(kTileE, nelem - e0), d0 = blockIdx.y * kTileD;
 #pragma unroll
-  for (int q = 0; q < NN * kTileE / 256; ++q) {
-    const int t = q * 256 + threadIdx.x, le = t >> 6, d = t & 63;
-    if (le < ne) tile[ad[d]][le] = in[(int64_t)e0 * NN + t];
+  for (int q = 0; q < kTileD * kTileE / 256; ++q) {
+    const int t = q * 256 + threadIdx.x, le = t / kTileD, d = t % kTileD;
+    if (le < ne) tile[d][le] = in[(int64_t)(e0 + le) * NN + d0 + d];
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < NN * kTileE / 256; ++q) {
-    const int t = q * 256 + threadIdx.x, le = t % kTileE, an = t / kTileE;
-    if (le < ne) ref[e0 + le + (int64_t)nelem * an] = tile[an][le];
+  for (int q = 0; q < kTileD * kTileE / 256; ++q) {
+    const int t = q * 256 + threadIdx.x, le = t % kTileE, d = t / kTileE;
+    if (le < ne) ref[e0 + le + (int64_t)nelem * perm.a[d0 + d]] = tile[d][le];
   }
 }
 
+static NodePerm node_perm(const SodMesh* m) {
+  NodePerm p;
+  for (int d = 0; d < NN; ++d) p.a[d] = m->perm_a_of_d[d];
+  return p;
+}
 int mesh_ref_to_internal_elem(SodMesh* m, const double* ref, double* out, cudaStream_t st, float* out32) {
-  k_ref2int<<<(m->nelem + kTileE - 1) / kTileE, 256, 0, st>>>(m->nelem, m->a_of_d_dev, ref, out, out32);
+  k_ref2int<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, node_perm(m), ref, out,
+                                                                                out32);
+  SOD_CHECK_LAUNCH();
+  return SOD_OK;
+}
+int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStream_t st) {
+  k_int2ref<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, node_perm(m), in, ref);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
 int mesh_mue_in(SodMesh* m, const double* mu_e, bool mixed, cudaStream_t st) {
   return mesh_ref_to_internal_elem(m, mu_e, m->mue_int, st, mixed ? m->mue32 : nullptr);
 }
-int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStream_t st) {
-  k_int2ref<<<(m->nelem + kTileE - 1) / kTileE, 256, 0, st>>>(m->nelem, m->a_of_d_dev, in, ref);
-  SOD_CHECK_LAUNCH();
-  return SOD_OK;
-}
-
 __global__ void k_inverse(int64_t n, const double* __restrict__ v, double* __restrict__ out) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) out[t] = 1.0 / v[t];
@@ -545,11 +550,9 @@ int sod_mesh_create(const SodMeshDesc* desc, const SodParams* params, SodMesh** 
   ALLOC(m->helem_l, sizeof(double) * E * NN);
   ALLOC(m->jratio, sizeof(double) * E);
   ALLOC(m->mue_int, sizeof(double) * E * NN);
-  ALLOC(m->a_of_d_dev, sizeof(int32_t) * NN);
   if (cudaMemcpy(m->econn, econn.data(), sizeof(int32_t) * E * NN, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(m->n2e_ptr, ptr.data(), sizeof(int32_t) * (N + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(m->n2e, idx.data(), sizeof(int32_t) * E * NN, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(m->a_of_d_dev, m->perm_a_of_d, sizeof(int32_t) * NN, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(m->mue_int, 0, sizeof(double) * E * NN) != cudaSuccess) {
     set_error("mesh upload failed: %s", cudaGetErrorString(cudaGetLastError()));
     return fail(SOD_ERR_CUDA);
