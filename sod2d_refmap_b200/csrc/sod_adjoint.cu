@@ -69,8 +69,8 @@ __device__ __forceinline__ void load4(const double* p, double (&w)[4]) {
 // the next in registers (up to 192 doubles) and spills them.
 __device__ __forceinline__ void pass_fence() { asm volatile("" ::: "memory"); }
 
-// Resident CTAs per SM the register budget must allow: 6 (168 registers, no spill) 0.282 ms for the whole
-// call at 32^3, 8 (128 registers, 92 bytes of spill) 0.297 ms.
+// Resident CTAs per SM the register budget must allow: 6 (168 registers, 48 bytes of spill, total enthalpy 4)
+// 172 us for the whole call at 27^3; 8 (128 registers) 206 us; 4 without spill 186 us.
 #ifndef SOD_VJP_MIN_BLOCKS
 #define SOD_VJP_MIN_BLOCKS 6
 #endif

@@ -54,6 +54,19 @@ static void free_state(SodState& s) {
     if (p) cudaFree(p);
 }
 
+// A member's columns (doubles, column lengths ddst and dsrc apart) as one strided copy: a copy per column of mu_e was
+// 64 synchronous calls.  Column by column only where a distance exceeds the largest pitch of a strided copy,
+// 2^31 - 1 bytes (more than 268 million nodes).
+static cudaError_t copy_columns(double* dst, int64_t ddst, const double* src, int64_t dsrc, int64_t len, int ncol,
+                                cudaMemcpyKind kind) {
+  constexpr int64_t kMaxPitch = (((int64_t)1 << 31) - 1) / (int64_t)sizeof(double);
+  if (ddst <= kMaxPitch && dsrc <= kMaxPitch)
+    return cudaMemcpy2D(dst, sizeof(double) * ddst, src, sizeof(double) * dsrc, sizeof(double) * len, ncol, kind);
+  for (int c = 0; c < ncol; ++c)
+    if (cudaError_t e = cudaMemcpy(dst + c * ddst, src + c * dsrc, sizeof(double) * len, kind)) return e;
+  return cudaSuccess;
+}
+
 extern "C" {
 
 void sod_batch_destroy(SodBatch* B) {
@@ -213,11 +226,11 @@ int sod_batch_set_member(SodBatch* B, int member, const SodState* h) {
   SOD_CUDA(cudaMemcpy(B->st.rho + no, h->rho, 8 * Ni, cudaMemcpyHostToDevice));
   SOD_CUDA(cudaMemcpy(B->st.E + no, h->E, 8 * Ni, cudaMemcpyHostToDevice));
   SOD_CUDA(cudaMemcpy(B->st.mu_factor + no, h->mu_factor, 8 * Ni, cudaMemcpyHostToDevice));
-  SOD_CUDA(cudaMemcpy2D(B->st.q + no, 8 * N, h->q, 8 * Ni, 8 * Ni, 3, cudaMemcpyHostToDevice));
-  if (h->u) SOD_CUDA(cudaMemcpy2D(B->st.u + no, 8 * N, h->u, 8 * Ni, 8 * Ni, 3, cudaMemcpyHostToDevice));
+  SOD_CUDA(copy_columns(B->st.q + no, N, h->q, Ni, Ni, 3, cudaMemcpyHostToDevice));
+  if (h->u) SOD_CUDA(copy_columns(B->st.u + no, N, h->u, Ni, Ni, 3, cudaMemcpyHostToDevice));
   if (h->csound) SOD_CUDA(cudaMemcpy(B->st.csound + no, h->csound, 8 * Ni, cudaMemcpyHostToDevice));
   if (h->mu_fluid) SOD_CUDA(cudaMemcpy(B->st.mu_fluid + no, h->mu_fluid, 8 * Ni, cudaMemcpyHostToDevice));
-  SOD_CUDA(cudaMemcpy2D(B->st.mu_e + eo, 8 * E, h->mu_e, 8 * Ei, 8 * Ei, NN, cudaMemcpyHostToDevice));
+  SOD_CUDA(copy_columns(B->st.mu_e + eo, E, h->mu_e, Ei, Ei, NN, cudaMemcpyHostToDevice));
   return SOD_OK;
 }
 
@@ -232,10 +245,9 @@ int sod_batch_get_member(SodBatch* B, int member, SodState* h) {
       {h->machno, B->st.machno}, {h->mu_fluid, B->st.mu_fluid}, {h->Reta, B->st.Reta}};
   for (auto& f : sc)
     if (f.hst) SOD_CUDA(cudaMemcpy(f.hst, f.dev + no, 8 * Ni, cudaMemcpyDeviceToHost));
-  // a member's columns as one strided copy each (a copy per column of mu_e was 64 synchronous calls)
-  if (h->q) SOD_CUDA(cudaMemcpy2D(h->q, 8 * Ni, B->st.q + no, 8 * N, 8 * Ni, 3, cudaMemcpyDeviceToHost));
-  if (h->u) SOD_CUDA(cudaMemcpy2D(h->u, 8 * Ni, B->st.u + no, 8 * N, 8 * Ni, 3, cudaMemcpyDeviceToHost));
-  if (h->mu_e) SOD_CUDA(cudaMemcpy2D(h->mu_e, 8 * Ei, B->st.mu_e + eo, 8 * E, 8 * Ei, NN, cudaMemcpyDeviceToHost));
+  if (h->q) SOD_CUDA(copy_columns(h->q, Ni, B->st.q + no, N, Ni, 3, cudaMemcpyDeviceToHost));
+  if (h->u) SOD_CUDA(copy_columns(h->u, Ni, B->st.u + no, N, Ni, 3, cudaMemcpyDeviceToHost));
+  if (h->mu_e) SOD_CUDA(copy_columns(h->mu_e, Ei, B->st.mu_e + eo, E, Ei, NN, cudaMemcpyDeviceToHost));
   return SOD_OK;
 }
 

@@ -47,7 +47,7 @@ constexpr int kBatch = 16;  // CG iterations per graph replay
 
 // device scalar slots
 enum {
-  S_Q1 = 0, S_T1, S_NUM, S_BETA, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD,
+  S_Q1 = 0, S_T1, S_BNORM2, S_TOL, S_ITER, S_MAXIT, S_DONE, S_Q1OLD,
   S_SKIP,  // S_DONE as the update kernel found it: the p update stores S_DONE, so none of its threads reads it
   S_COUNT
 };
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_pupdate(int n, double* scal, cons
   sum_partials<3>(part, stride, npart, t3);
   const double beta_d = t3[1] / scal[S_Q1OLD];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    scal[S_T1] = t3[0]; scal[S_NUM] = t3[1]; scal[S_BETA] = beta_d; scal[S_Q1] = t3[2];
+    scal[S_T1] = t3[0]; scal[S_Q1] = t3[2];
     const double it = scal[S_ITER] + 1.0;
     scal[S_ITER] = it;
     if (sqrt(t3[0]) < scal[S_TOL] * sqrt(scal[S_BNORM2]) || it >= scal[S_MAXIT]) scal[S_DONE] = 1.0;

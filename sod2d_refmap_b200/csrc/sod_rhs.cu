@@ -41,12 +41,11 @@
 namespace sod {
 
 // weak divergence sum_dir sum_m D[m][idx_dir] V_dir(line point m)
-template <typename R>
-__device__ __forceinline__ R divT(const R* fx, const R* fy, const R* fz, int i, int j, int k, const R* DTx,
-                                  const R* DTy, const R* DTz) {
-  const R* ax = fx + 4 * j + PLANE * k;
-  const R* ay = fy + i + PLANE * k;
-  const R* az = fz + i + 4 * j;
+__device__ __forceinline__ double divT(const double* fx, const double* fy, const double* fz, int i, int j, int k, const double* DTx,
+                                  const double* DTy, const double* DTz) {
+  const double* ax = fx + 4 * j + PLANE * k;
+  const double* ay = fy + i + PLANE * k;
+  const double* az = fz + i + 4 * j;
   return DTx[0] * ax[0] + DTx[1] * ax[1] + DTx[2] * ax[2] + DTx[3] * ax[3] +
          (DTy[0] * ay[0] + DTy[1] * ay[4] + DTy[2] * ay[8] + DTy[3] * ay[12]) +
          (DTz[0] * az[0] + DTz[1] * az[PLANE] + DTz[2] * az[2 * PLANE] + DTz[3] * az[3 * PLANE]);
@@ -56,17 +55,15 @@ constexpr int NBUF = 8;  // rho, u0, u1, u2, H, eta, p, T
 constexpr int NP2 = 18;  // 6 contravariant fluxes x 3 directions
 constexpr int NDTAB = 36;  // per CTA: D rows, then D^T rows, then D's row sums
 
-template <typename R>
 constexpr size_t rhs_smem_bytes(int epb) {
-  return sizeof(R) * (NDTAB + (size_t)epb * (NBUF + NP2) * FSTRIDE);
+  return sizeof(double) * (NDTAB + (size_t)epb * (NBUF + NP2) * FSTRIDE);
 }
 
 // One tile of EPB elements (64 threads each) of the fused RHS; smem_raw holds
-// rhs_smem_bytes<R>(EPB).  Every thread of the block calls it (it holds block barriers).
+// rhs_smem_bytes(EPB).  Every thread of the block calls it (it holds block barriers).
 // TOTH: flag_total_enthalpy (energy convection of full_convec_ijk_H)
-template <typename R, int EPB, bool TOTH>
+template <int EPB, bool TOTH>
 __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsigned char* smem_raw) {
-  static_assert(sizeof(R) == 8, "FP64");
   double* dtab = reinterpret_cast<double*>(smem_raw);
   const int tid = threadIdx.x;
   const int es = tid >> 6;
@@ -260,10 +257,10 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
 #ifndef SOD_KR64_MIN_CTAS
 #define SOD_KR64_MIN_CTAS 8
 #endif
-template <typename R, int EPB, bool TOTH>
+template <int EPB, bool TOTH>
 __global__ void __launch_bounds__(64 * EPB, (EPB >= SOD_KR64_MIN_CTAS ? 1 : SOD_KR64_MIN_CTAS / EPB)) k_rhs_fused(const RhsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  rhs_fused_tile<R, EPB, TOTH>(a, blockIdx.x, smem_raw);
+  rhs_fused_tile<EPB, TOTH>(a, blockIdx.x, smem_raw);
 }
 
 // One RK stage of the FP64 path in one cooperative launch (persistent blocks): the fused RHS
@@ -274,7 +271,7 @@ __global__ void __launch_bounds__(64 * EPB) k_stage_fused(const StageArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ntiles = (p.r.nelem + EPB - 1) / EPB;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    rhs_fused_tile<double, EPB, TOTH>(p.r, t, smem_raw);
+    rhs_fused_tile<EPB, TOTH>(p.r, t, smem_raw);
     __syncthreads();  // the next tile reuses the shared memory
   }
   persist_stage_tail<double, EPB>(p, smem_raw);
@@ -333,16 +330,16 @@ __global__ void __launch_bounds__(32 * KV_WARPS, SOD_KV_MIN_BLOCKS) k_visc_dt(co
 // ---------------------------------------------------------------------------------------------
 // Host-side launch helpers
 // ---------------------------------------------------------------------------------------------
-template <typename R, int EPB>
+template <int EPB>
 static int set_rhs_attr() {
-  SOD_CUDA(cudaFuncSetAttribute(k_rhs_fused<R, EPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rhs_smem_bytes<R>(EPB)));
-  SOD_CUDA(cudaFuncSetAttribute(k_rhs_fused<R, EPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rhs_smem_bytes<R>(EPB)));
+  SOD_CUDA(cudaFuncSetAttribute(k_rhs_fused<EPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)rhs_smem_bytes(EPB)));
+  SOD_CUDA(cudaFuncSetAttribute(k_rhs_fused<EPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)rhs_smem_bytes(EPB)));
   SOD_CUDA(cudaFuncSetAttribute(k_stage_fused<EPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rhs_smem_bytes<double>(EPB)));
+                                (int)rhs_smem_bytes(EPB)));
   SOD_CUDA(cudaFuncSetAttribute(k_stage_fused<EPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rhs_smem_bytes<double>(EPB)));
+                                (int)rhs_smem_bytes(EPB)));
   return SOD_OK;
 }
 
@@ -351,7 +348,7 @@ template <int EPB>
 static int launch_stage_fused_t(const StageArgs& p, int ctas_per_sm, int* grid_out, cudaStream_t st) {
   const bool toth = p.r.prm.total_enthalpy != 0;
   const void* fn = toth ? (const void*)k_stage_fused<EPB, true> : (const void*)k_stage_fused<EPB, false>;
-  const size_t smem = rhs_smem_bytes<double>(EPB);
+  const size_t smem = rhs_smem_bytes(EPB);
   int occ = 0, dev = 0, nsm = 0;
   SOD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 64 * EPB, smem));
   SOD_CUDA(cudaGetDevice(&dev));
@@ -395,7 +392,7 @@ void persist_kernel_info(bool mixed, int epb, bool toth, const void** fn, size_t
     case 8: *fn = toth ? (const void*)k_stage_fused<8, true> : (const void*)k_stage_fused<8, false>; break;
     default: *fn = toth ? (const void*)k_stage_fused<2, true> : (const void*)k_stage_fused<2, false>; epb = 2;
   }
-  *smem = rhs_smem_bytes<double>(epb);
+  *smem = rhs_smem_bytes(epb);
 }
 
 // One persistent stage launch of either precision
@@ -412,22 +409,22 @@ int launch_stage(const StageArgs& p, bool mixed, int epb, int ctas_per_sm, int* 
 int init_kernel_attrs() {
   static bool done = false;
   if (done) return SOD_OK;
-  int rc = set_rhs_attr<double, 1>() | set_rhs_attr<double, 2>() | set_rhs_attr<double, 4>() |
-           set_rhs_attr<double, 8>() |
+  int rc = set_rhs_attr<1>() | set_rhs_attr<2>() | set_rhs_attr<4>() |
+           set_rhs_attr<8>() |
            init_rhs_mixed2_attrs();
   if (rc) return SOD_ERR_CUDA;
   done = true;
   return SOD_OK;
 }
 
-template <typename R, int EPB>
+template <int EPB>
 static int launch_rhs_t(const RhsArgs& a, cudaStream_t st) {
-  const size_t smem = rhs_smem_bytes<R>(EPB);
+  const size_t smem = rhs_smem_bytes(EPB);
   const int grid = (a.nelem + EPB - 1) / EPB;
   if (a.prm.total_enthalpy)
-    k_rhs_fused<R, EPB, true><<<grid, 64 * EPB, smem, st>>>(a);
+    k_rhs_fused<EPB, true><<<grid, 64 * EPB, smem, st>>>(a);
   else
-    k_rhs_fused<R, EPB, false><<<grid, 64 * EPB, smem, st>>>(a);
+    k_rhs_fused<EPB, false><<<grid, 64 * EPB, smem, st>>>(a);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
@@ -457,10 +454,10 @@ int launch_rhs(SodMesh* m, bool mixed, int epb, const double* rho, const double*
   const RhsArgs a = make_rhs_args(m, mixed, rho, q0, q1, q2, E, mu_factor, musgs_int);
   if (!mixed) {
     switch (epb) {
-      case 1: return launch_rhs_t<double, 1>(a, st);
-      case 4: return launch_rhs_t<double, 4>(a, st);
-      case 8: return launch_rhs_t<double, 8>(a, st);
-      default: return launch_rhs_t<double, 2>(a, st);
+      case 1: return launch_rhs_t<1>(a, st);
+      case 4: return launch_rhs_t<4>(a, st);
+      case 8: return launch_rhs_t<8>(a, st);
+      default: return launch_rhs_t<2>(a, st);
     }
   } else {
     return launch_rhs_mixed2(a, epb, st);

@@ -41,7 +41,7 @@ struct GatherArgs {
   double* scal;             // [0] eta mean, [1] eta norm
   int normalise;
   double* dt_bits;          // stage 4: preset for the time-step reduction that follows it
-  int ndt;                  // its length (1, or the ensemble's members; 0: not preset)
+  int ndt;                  // its length (1, or the ensemble's members)
   const double* src;        // momentum source term (npoin,3) or null
   const double* wm;         // wall-model momentum terms (npoin,3) or null
 };
