@@ -18,7 +18,7 @@
 // The same pass structure gives the forward gradients and the D-line sums of the seeds (the
 // transpose of pass 2's D^T); the viscous stress is reversed pointwise and its five gradient
 // fields (u, rho, T) go back through He^T and D^T.  32^3, one launch: 218 us; 467 us with the 29 nodal
-// product fields each sent back through three line arrays.  Bounded by the L1 data pipe (81% busy)
+// product fields each sent back through three line arrays.  Bounded by the L1 data pipe (80% busy)
 // and the FP64 pipe (60%) at 12 resident warps per SM (168 registers); 16 warps (128 registers, own
 // values parked in shared memory) measured 206 us against 173 us for the call at 27^3.
 // Element-node adjoints are assembled by the same ordered CSR gather as the forward path.

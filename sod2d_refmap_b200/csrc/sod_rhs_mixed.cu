@@ -30,7 +30,7 @@
 //
 // Measured at 64^3 (262,144 elements, one launch): 0.827 ms, 1.254 ms with the 12 gradient fields
 // and 25 staged-factor products of the quartets formed one by one.  Bounded by latency at 20
-// resident warps per SM with the L1 data pipe ~70% and the issue slots ~55% busy; HBM floor 0.24 ms.
+// resident warps per SM with the L1 data pipe ~70% and the issue slots ~60% busy; HBM floor 0.24 ms.
 //
 // Precision.  div u cancels by orders of magnitude and multiplies rho, H and eta, so its line sums and
 // fold run in FP64.  The viscous terms differentiate twice, so an error in a gradient is raised by the
