@@ -144,6 +144,7 @@ int sod_batch_create(SodMesh* const* meshes, int nmesh, SodBatch** out) {
   std::memcpy(m->wgp_nat, m0->wgp_nat, sizeof(m->wgp_nat));
   std::memcpy(m->perm_a_of_d, m0->perm_a_of_d, sizeof(m->perm_a_of_d));
   std::memcpy(m->perm_d_of_a, m0->perm_d_of_a, sizeof(m->perm_d_of_a));
+  mesh_set_kernel_tables(m);
   m->nmember = nmesh;
   auto fail = [&](const char* what) {
     set_error("sod_batch_create: %s", what);

@@ -92,14 +92,10 @@ struct DevParams {
 struct DMat {
   double d[NP1][NP1];
 };
-// Row sums of D: zero but for the rounding of its entries (as given by the caller), to double precision.
-inline void d_row_sums(const DMat& D, double (&s)[NP1]) {
-  for (int r = 0; r < NP1; ++r) {
-    long double t = 0.0L;
-    for (int c = 0; c < NP1; ++c) t += D.d[r][c];
-    s[r] = (double)t;
-  }
-}
+// internal node order of an element, as a kernel parameter
+struct NodePerm {
+  unsigned char a[NN];  // reference node of internal node d
+};
 
 // Arguments of the fused element-RHS kernels.
 struct RhsArgs {
@@ -116,8 +112,10 @@ struct RhsArgs {
   const double* __restrict__ mu_factor;  // per node
   void* rel;                       // R [(e*64 + d)*6 + f]
   DMat D;
-  double Dsum[NP1];                // row sums of D (FP64 kernels)
-  float Df[NP1][NP1];              // D in FP32 (mixed kernels)
+  union {
+    double Dsum[NP1];              // row sums of D (FP64 kernels)
+    float Df[NP1][NP1];            // D in FP32 (mixed kernels)
+  };
   DevParams prm;
 };
 
@@ -304,6 +302,8 @@ struct SodMesh {
   int device = 0;
   sod::DevParams prm{};
   sod::DMat D{};
+  double Dsum[sod::NP1];            // row sums of D: zero but for the rounding of its entries
+  sod::NodePerm node_perm;          // perm_a_of_d
   double wgp_nat[sod::NN];
   int perm_a_of_d[sod::NN];   // reference local node a of library node d
   int perm_d_of_a[sod::NN];
@@ -370,6 +370,8 @@ int mesh_from_device_ref(int nelem, int npoin, int base, const int32_t* connec, 
                          const SodParams* params, cudaStream_t st, SodMesh** out);
 // scalars, counters and 1 / Ml of a mesh whose Ml is set (on the default stream; the caller waits)
 int mesh_init_node_data(SodMesh* m);
+// Dsum and node_perm of a mesh whose D and perm_a_of_d are set
+void mesh_set_kernel_tables(SodMesh* m);
 // f32_copy (optional): FP32 copy of the internal array
 int mesh_ref_to_internal_elem(SodMesh* m, const double* ref_dev /*(nelem,64) F*/, double* int_dev,
                               cudaStream_t st, float* f32_copy = nullptr);

@@ -194,9 +194,6 @@ int launch_copy_f32(const double* src, float* dst, int64_t n, cudaStream_t st) {
 // copy) / out, us: 4^3 1.8 / 1.7, 24^3 3.6 / 3.2, 64^3 (134 MB each way) 54 / 37; a thread per value
 // (copy apart) 3.6 / 1.8, 9.7 / 7.6, 113 / 112; tiles of 64 nodes 2.5 / 2.1, 3.6 / 3.5, 54 / 39.
 constexpr int kTileE = 32, kTileD = 32;
-struct NodePerm {
-  int a[NN];  // reference node of internal node d
-};
 __global__ void __launch_bounds__(256) k_ref2int(int nelem, const __grid_constant__ NodePerm perm,
                                                  const double* __restrict__ ref, double* __restrict__ out,
                                                  float* __restrict__ out32) {
@@ -236,19 +233,14 @@ __global__ void __launch_bounds__(256) k_int2ref(int nelem, const __grid_constan
   }
 }
 
-static NodePerm node_perm(const SodMesh* m) {
-  NodePerm p;
-  for (int d = 0; d < NN; ++d) p.a[d] = m->perm_a_of_d[d];
-  return p;
-}
 int mesh_ref_to_internal_elem(SodMesh* m, const double* ref, double* out, cudaStream_t st, float* out32) {
-  k_ref2int<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, node_perm(m), ref, out,
+  k_ref2int<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, m->node_perm, ref, out,
                                                                                 out32);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
 int mesh_internal_to_ref_elem(SodMesh* m, const double* in, double* ref, cudaStream_t st) {
-  k_int2ref<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, node_perm(m), in, ref);
+  k_int2ref<<<dim3((m->nelem + kTileE - 1) / kTileE, NN / kTileD), 256, 0, st>>>(m->nelem, m->node_perm, in, ref);
   SOD_CHECK_LAUNCH();
   return SOD_OK;
 }
@@ -258,6 +250,16 @@ int mesh_mue_in(SodMesh* m, const double* mu_e, bool mixed, cudaStream_t st) {
 __global__ void k_inverse(int64_t n, const double* __restrict__ v, double* __restrict__ out) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) out[t] = 1.0 / v[t];
+}
+
+// what the kernels are given of D and of the node order, formed once
+void mesh_set_kernel_tables(SodMesh* m) {
+  for (int r = 0; r < NP1; ++r) {
+    long double t = 0.0L;
+    for (int c = 0; c < NP1; ++c) t += m->D.d[r][c];
+    m->Dsum[r] = (double)t;
+  }
+  for (int d = 0; d < NN; ++d) m->node_perm.a[d] = (unsigned char)m->perm_a_of_d[d];
 }
 
 // Local node order of the library (natural d = i + 4j + 16k) from the reference's gmshAtoI/J/K
@@ -288,6 +290,7 @@ int mesh_set_local_tables(SodMesh* m, const int32_t* gI, const int32_t* gJ, cons
   }
   if (wgp)
     for (int d = 0; d < NN; ++d) m->wgp_nat[d] = wgp[m->perm_a_of_d[d]];
+  mesh_set_kernel_tables(m);
   return SOD_OK;
 }
 

@@ -441,9 +441,11 @@ static RhsArgs make_rhs_args(SodMesh* m, bool mixed, const double* rho, const do
   a.mu_factor = mu_factor;
   a.rel = m->buf.rel;
   a.D = m->D;
-  d_row_sums(m->D, a.Dsum);
-  for (int r = 0; r < NP1; ++r)
-    for (int c = 0; c < NP1; ++c) a.Df[r][c] = (float)m->D.d[r][c];
+  for (int r = 0; r < NP1; ++r) {
+    if (!mixed) a.Dsum[r] = m->Dsum[r];
+    else
+      for (int c = 0; c < NP1; ++c) a.Df[r][c] = (float)m->D.d[r][c];
+  }
   a.prm = m->prm;
   return a;
 }

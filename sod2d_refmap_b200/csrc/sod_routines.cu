@@ -35,18 +35,27 @@ __device__ __forceinline__ Point point_of(int lt) {
   return p;
 }
 
+// Each kernel is given what it reads: on a small mesh a call is bound by the host's launches, and one struct
+// for all with D's row sums in it (312 bytes) cost up to 0.3 us a call.
 struct RefArgs {
-  int nelem;
   int64_t npoin;
   const int32_t* econn;
   const double* geo;
+  double* rel;                                  // rows [(e*64 + d)*6 + f]
   DMat D;
+  const double* u;
+};
+struct ConvecArgs : RefArgs {
+  const double *q, *rho, *pr, *E;
   double Dsum[NP1];                             // row sums of D
-  const double *u, *q, *rho, *pr, *E;          // convec / scalar
-  const double *rho_n, *Tem, *mu_fluid;         // diffusion
+};
+struct ScalarArgs : RefArgs {
+  const double *q, *eta;
+};
+struct DiffusionArgs : RefArgs {
+  const double *rho, *rho_n, *Tem, *mu_fluid;
   const double *mue, *musgs;                    // internal layout [e][64]
   double Cp, Pr, c_rho, c_ener;
-  double* rel;                                  // rows [(e*64 + d)*6 + f]
 };
 
 // full_convec_ijk (elem_convec.f90:241-435); TOTH: full_convec_ijk_H (elem_convec.f90:48-187),
@@ -62,7 +71,7 @@ struct RefArgs {
 // 2.3e-16, with whole values in the sums 7.4e-15, 1.2e-14 and 3.3e-16 (and 24 us instead of 27 at 20^3).  On white
 // noise, where differences are no smaller than values, momentum 2.5e-16 (quartets 1.8e-16).
 template <bool TOTH>
-__global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefArgs a) {
+__global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ ConvecArgs a) {
   constexpr int F_K = TOTH ? 8 : 9;         // k, after
   __shared__ double f[F_K + 1][FSTRIDE];   // rho, p, E (TOTH: p + E), u, q
   __shared__ double Ds[16], Dsum[NP1];
@@ -155,7 +164,7 @@ __global__ void __launch_bounds__(64) k_convec_ref(const __grid_constant__ RefAr
 }
 
 // generic_scalar_convec_ijk (elem_convec.f90:488-556)
-__global__ void __launch_bounds__(64) k_scalar_ref(const __grid_constant__ RefArgs a) {
+__global__ void __launch_bounds__(64) k_scalar_ref(const __grid_constant__ ScalarArgs a) {
   __shared__ double f[7][FSTRIDE];
   __shared__ double Ds[16];
   const int e = blockIdx.x;
@@ -171,7 +180,7 @@ __global__ void __launch_bounds__(64) k_scalar_ref(const __grid_constant__ RefAr
   double u[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) { u[c] = a.u[n + N * c]; f[1 + c][p.s] = u[c]; f[4 + c][p.s] = a.q[n + N * c]; }
-  const double eta = a.E[n];
+  const double eta = a.eta[n];
   f[0][p.s] = eta;
   __syncthreads();
   double div = 0.0, divU = 0.0, adv = 0.0;
@@ -197,7 +206,7 @@ __global__ void __launch_bounds__(64) k_scalar_ref(const __grid_constant__ RefAr
 }
 
 // full_diffusion_ijk (elem_diffu.f90:44-194)
-__global__ void __launch_bounds__(64) k_diffusion_ref(const __grid_constant__ RefArgs a) {
+__global__ void __launch_bounds__(64) k_diffusion_ref(const __grid_constant__ DiffusionArgs a) {
   __shared__ double f[5][FSTRIDE];  // rho, T, u
   __shared__ double V[18][FSTRIDE];
   __shared__ double Ds[16], DTs[16];
@@ -412,17 +421,22 @@ static int gather_out(SodMesh* m, double* Rmass, double* Rmom, double* Rener, cu
   return SOD_OK;
 }
 
-static RefArgs ref_args(SodMesh* m) {
-  RefArgs a{};
-  a.nelem = m->nelem;
+template <typename Args>
+static Args ref_args(SodMesh* m, const double* u) {
+  Args a{};
   a.npoin = m->npoin;
   a.econn = m->econn;
   a.geo = m->geo64;
-  a.D = m->D;
-  d_row_sums(m->D, a.Dsum);
   a.rel = (double*)m->buf.rel;
-  a.c_rho = m->prm.c_rho;
-  a.c_ener = m->prm.c_ener;
+  a.D = m->D;
+  a.u = u;
+  return a;
+}
+static ConvecArgs convec_args(SodMesh* m, const double* u, const double* q, const double* rho, const double* pr,
+                              const double* E) {
+  ConvecArgs a = ref_args<ConvecArgs>(m, u);
+  a.q = q; a.rho = rho; a.pr = pr; a.E = E;
+  for (int r = 0; r < NP1; ++r) a.Dsum[r] = m->Dsum[r];
   return a;
 }
 
@@ -438,9 +452,7 @@ int sod_full_convec_ijk(SodMesh* m, const double* u, const double* q, const doub
   cudaStream_t st = (cudaStream_t)stream;
   int rc = ensure_step_buffers(m, false);
   if (rc) return rc;
-  RefArgs a = ref_args(m);
-  a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E;
-  k_convec_ref<false><<<m->nelem, 64, 0, st>>>(a);
+  k_convec_ref<false><<<m->nelem, 64, 0, st>>>(convec_args(m, u, q, rho, pr, E));
   SOD_CHECK_LAUNCH();
   return gather_out(m, Rmass, Rmom, Rener, st);
 }
@@ -451,9 +463,7 @@ int sod_full_convec_ijk_H(SodMesh* m, const double* u, const double* q, const do
   cudaStream_t st = (cudaStream_t)stream;
   int rc = ensure_step_buffers(m, false);
   if (rc) return rc;
-  RefArgs a = ref_args(m);
-  a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E;
-  k_convec_ref<true><<<m->nelem, 64, 0, st>>>(a);
+  k_convec_ref<true><<<m->nelem, 64, 0, st>>>(convec_args(m, u, q, rho, pr, E));
   SOD_CHECK_LAUNCH();
   return gather_out(m, Rmass, Rmom, Rener, st);
 }
@@ -464,8 +474,8 @@ int sod_generic_scalar_convec_ijk(SodMesh* m, const double* q, const double* eta
   cudaStream_t st = (cudaStream_t)stream;
   int rc = ensure_step_buffers(m, false);
   if (rc) return rc;
-  RefArgs a = ref_args(m);
-  a.u = u; a.q = q; a.E = eta;
+  ScalarArgs a = ref_args<ScalarArgs>(m, u);
+  a.q = q; a.eta = eta;
   k_scalar_ref<<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
   k_gather_one<<<(m->npoin + 255) / 256, 256, 0, st>>>(m->npoin, m->n2e_ptr, m->n2e, (const double*)m->buf.rel, Rconvec);
@@ -489,8 +499,9 @@ int sod_full_diffusion_ijk(SodMesh* m, double Cp, double Pr, const double* rho_n
     rc = mesh_ref_to_internal_elem(m, mu_sgs, musgs_int, st);
     if (rc) return rc;
   }
-  RefArgs a = ref_args(m);
-  a.rho_n = rho_n; a.rho = rho; a.u = u; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mue = m->mue_int; a.musgs = musgs_int;
+  DiffusionArgs a = ref_args<DiffusionArgs>(m, u);
+  a.c_rho = m->prm.c_rho; a.c_ener = m->prm.c_ener;
+  a.rho_n = rho_n; a.rho = rho; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mue = m->mue_int; a.musgs = musgs_int;
   a.Cp = Cp; a.Pr = Pr;
   k_diffusion_ref<<<m->nelem, 64, 0, st>>>(a);
   SOD_CHECK_LAUNCH();
