@@ -25,6 +25,8 @@ def _torch():
 
 
 def _ptr(t) -> int:
+    # plain int: the entries' argtypes convert it (a c_void_p of its own per argument costs 0.13 us each, and
+    # calls on small meshes are bound by the host)
     return 0 if t is None else int(t.data_ptr())
 
 
@@ -358,7 +360,7 @@ class Sod2dMesh:
         lv = None if leviCivi is None else np.asfortranarray(leviCivi, dtype=np.float64).ravel(order="F")
         _lib.check(_lib.load().sod_compute_field_derivs(
             self.handle, C.c_void_p(_ptr(_contig(rho))), C.c_void_p(_ptr(_contig(u))),
-            _np_ptr(lv) if lv is not None else None, *(C.c_void_p(_ptr(t)) for t in (g, c, dv, qc)), _stream(stream)))
+            _np_ptr(lv) if lv is not None else None, *[_ptr(t) for t in (g, c, dv, qc)], _stream(stream)))
         return g, c, dv, qc
 
     def set_rhs_config(self, precision: int, config: int):
@@ -372,9 +374,9 @@ class Sod2dMesh:
                    Rmom=torch.zeros(3, N, dtype=torch.float64, device="cuda"),
                    Rener=torch.zeros(N, dtype=torch.float64, device="cuda"),
                    Reta=torch.zeros(N, dtype=torch.float64, device="cuda"))
-        _lib.check(_lib.load().sod_rhs(self.handle, *(C.c_void_p(_ptr(t)) for t in (
+        _lib.check(_lib.load().sod_rhs(self.handle, *[_ptr(t) for t in (
             state.rho, state.q, state.E, state.mu_e, state.mu_factor, out["Rmass"], out["Rmom"], out["Rener"],
-            out["Reta"])), int(precision), _stream(stream)))
+            out["Reta"])], int(precision), _stream(stream)))
         return out
 
     def tgv_diagnostics(self, state: Sod2dState, rho0: float, volT: float = 0.0, stream=None) -> dict:
@@ -382,8 +384,8 @@ class Sod2dMesh:
         the summed gpvol)."""
         torch = _torch()
         out = torch.zeros(5, dtype=torch.float64, device="cuda")
-        _lib.check(_lib.load().sod_tgv_diagnostics(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            state.rho, state.u, state.mu_fluid, state.mu_e)), C.c_double(rho0), C.c_double(volT),
+        _lib.check(_lib.load().sod_tgv_diagnostics(self.handle, *[_ptr(t) for t in (
+            state.rho, state.u, state.mu_fluid, state.mu_e)], C.c_double(rho0), C.c_double(volT),
             C.c_void_p(_ptr(out)), _stream(stream)))
         v = out.cpu().tolist()
         return {"EK": v[0], "eps_S": v[1], "eps_D": v[2], "eps_T": v[3], "volT": v[4]}
@@ -397,7 +399,7 @@ class Sod2dMesh:
         g_q = torch.empty(3, N, dtype=torch.float64, device="cuda")
         g_E = torch.empty(N, dtype=torch.float64, device="cuda")
         args = [_contig(t) for t in (rho, q, E, mu_e, mu_factor, bar_Rmass, bar_Rmom, bar_Rener)]
-        _lib.check(_lib.load().sod_rhs_vjp(self.handle, *(C.c_void_p(_ptr(t)) for t in args + [g_rho, g_q, g_E]),
+        _lib.check(_lib.load().sod_rhs_vjp(self.handle, *[_ptr(t) for t in args + [g_rho, g_q, g_E]],
                                            _stream(stream)))
         return g_rho, g_q, g_E
 
@@ -425,13 +427,13 @@ class Sod2dMesh:
         args += [_contig(t) for t in (mu_factor, dt)]
         args += [None if stages is None else _contig(stages)]
         args += [_contig(t) for t in (bar_rho, bar_q, bar_E)]
-        _lib.check(_lib.load().sod_rk4_step_vjp(self.handle, *(C.c_void_p(_ptr(t)) for t in args + list(out)),
+        _lib.check(_lib.load().sod_rk4_step_vjp(self.handle, *[_ptr(t) for t in args + list(out)],
                                                 _stream(stream)))
         return out
 
     def adapt_dt(self, state: Sod2dState, stream=None):
-        _lib.check(_lib.load().sod_adapt_dt_cfl(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            state.u, state.csound, state.mu_fluid)), C.c_void_p(0), C.c_void_p(_ptr(state.rho)),
+        _lib.check(_lib.load().sod_adapt_dt_cfl(self.handle, *[_ptr(t) for t in (
+            state.u, state.csound, state.mu_fluid)], C.c_void_p(0), C.c_void_p(_ptr(state.rho)),
             C.c_void_p(_ptr(state.dt)), _stream(stream)))
         return state.dt
 
@@ -442,8 +444,8 @@ class Sod2dMesh:
         Rm = torch.empty(N, dtype=torch.float64, device="cuda")
         Rmo = torch.empty(3, N, dtype=torch.float64, device="cuda")
         Re = torch.empty(N, dtype=torch.float64, device="cuda")
-        _lib.check(_lib.load().sod_full_convec_ijk(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            u, q, rho, pr, E, Rm, Rmo, Re)), _stream(stream)))
+        _lib.check(_lib.load().sod_full_convec_ijk(self.handle, *[_ptr(t) for t in (
+            u, q, rho, pr, E, Rm, Rmo, Re)], _stream(stream)))
         return Rm, Rmo, Re
 
     def full_convec_ijk_H(self, u, q, rho, pr, E, stream=None):
@@ -453,15 +455,15 @@ class Sod2dMesh:
         Rm = torch.empty(N, dtype=torch.float64, device="cuda")
         Rmo = torch.empty(3, N, dtype=torch.float64, device="cuda")
         Re = torch.empty(N, dtype=torch.float64, device="cuda")
-        _lib.check(_lib.load().sod_full_convec_ijk_H(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            u, q, rho, pr, E, Rm, Rmo, Re)), _stream(stream)))
+        _lib.check(_lib.load().sod_full_convec_ijk_H(self.handle, *[_ptr(t) for t in (
+            u, q, rho, pr, E, Rm, Rmo, Re)], _stream(stream)))
         return Rm, Rmo, Re
 
     def generic_scalar_convec_ijk(self, f, eta, u, stream=None):
         torch = _torch()
         R = torch.empty(self.npoin, dtype=torch.float64, device="cuda")
-        _lib.check(_lib.load().sod_generic_scalar_convec_ijk(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            f, eta, u, R)), _stream(stream)))
+        _lib.check(_lib.load().sod_generic_scalar_convec_ijk(self.handle, *[_ptr(t) for t in (
+            f, eta, u, R)], _stream(stream)))
         return R
 
     def full_diffusion_ijk(self, rho_n, rho, u, Tem, mu_fluid, mu_e, mu_sgs=None, stream=None):
@@ -471,8 +473,8 @@ class Sod2dMesh:
         Rmo = torch.empty(3, N, dtype=torch.float64, device="cuda")
         Re = torch.empty(N, dtype=torch.float64, device="cuda")
         _lib.check(_lib.load().sod_full_diffusion_ijk(self.handle, C.c_double(self.prm.Cp), C.c_double(self.prm.Prt),
-                                                     *(C.c_void_p(_ptr(t)) for t in (rho_n, rho, u, Tem, mu_fluid,
-                                                                                     mu_e, mu_sgs, Rm, Rmo, Re)),
+                                                     *[_ptr(t) for t in (rho_n, rho, u, Tem, mu_fluid,
+                                                                                     mu_e, mu_sgs, Rm, Rmo, Re)],
                                                      _stream(stream)))
         return Rm, Rmo, Re
 
@@ -484,8 +486,8 @@ class Sod2dMesh:
     def smart_visc_spectral(self, Reta, rho, u, csound, Tem, eta, stream=None):
         torch = _torch()
         mu_e = torch.zeros(64, self.nelem, dtype=torch.float64, device="cuda")
-        _lib.check(_lib.load().sod_smart_visc_spectral(self.handle, *(C.c_void_p(_ptr(t)) for t in (
-            Reta, rho, u, csound, Tem, eta, mu_e)), _stream(stream)))
+        _lib.check(_lib.load().sod_smart_visc_spectral(self.handle, *[_ptr(t) for t in (
+            Reta, rho, u, csound, Tem, eta, mu_e)], _stream(stream)))
         return mu_e
 
 
@@ -500,8 +502,8 @@ def sutherland_viscosity(Tem, mu_factor, stream=None):
 def csr_spmv_scal(rdom, cdom, Mc, v, stream=None):
     torch = _torch()
     u = torch.empty(rdom.numel() - 1, dtype=torch.float64, device="cuda")
-    _lib.check(_lib.load().sod_csr_spmv_scal(int(u.numel()), int(Mc.numel()), *(C.c_void_p(_ptr(t)) for t in (
-        rdom, cdom, Mc, v, u)), _stream(stream)))
+    _lib.check(_lib.load().sod_csr_spmv_scal(int(u.numel()), int(Mc.numel()), *[_ptr(t) for t in (
+        rdom, cdom, Mc, v, u)], _stream(stream)))
     return u
 
 
@@ -656,7 +658,7 @@ def _legacy_call(fn_name: str, connec, Ngp, gpcar, gpvol, fields, out_shape):
     npoin = out_shape[0]
     R = torch.zeros(int(np.prod(out_shape)), dtype=torch.float64, device="cuda")
     _lib.check(getattr(_lib.load(), fn_name)(nelem, ngaus, npoin, nnode, ndime,
-                                             *(C.c_void_p(_ptr(t)) for t in args + [R]), _stream(None)))
+                                             *[_ptr(t) for t in args + [R]], _stream(None)))
     return R.cpu().numpy().reshape(out_shape, order="F")
 
 
@@ -683,7 +685,7 @@ def legacy_mom_diffusion(connec, Ngp, gpcar, gpvol, u, mu_e):
 
 # ---- the reference's subroutines with their complete argument lists (device arrays) ----------
 def _ptrs(*ts):
-    return [C.c_void_p(_ptr(t)) for t in ts]
+    return [_ptr(t) for t in ts]
 
 
 def full_convec_ijk_ref(nelem, npoin, connec, Ngp, dNgp, He, gpvol, dlxigp_ip, xgp, invAtoIJK, gmshAtoI, gmshAtoJ,
