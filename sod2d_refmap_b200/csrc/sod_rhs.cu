@@ -19,7 +19,7 @@
 //   mass      Rm = rho div u + sum_dir sum_m D[x][m] V^ drho
 //   f         f_x Rm + sum_dir sum_m D[x][m] V^ r^ df        f = u_c, H = h + k
 //   entropy   eta div u + sum_dir sum_m D[x][m] V^ deta
-//   (E+p)     G div u + sum_dir sum_m D[x][m] V^ dG          G = rho H, flag_total_enthalpy
+//   (E+p)     G div u + sum_dir sum_m D[x][m] V^ dG          G = E + p, flag_total_enthalpy
 // (the energy is linear in (h, k) and every h term has a k twin, so both quartets are evaluated on
 // H).  These are the reference's sums with the products expanded around the output point, where
 // the constant parts vanish but for the row sums of D (its rounding), which are counted: 19 FP64 operations
@@ -51,7 +51,7 @@ __device__ __forceinline__ double divT(const double* fx, const double* fy, const
          (DTz[0] * az[0] + DTz[1] * az[PLANE] + DTz[2] * az[2 * PLANE] + DTz[3] * az[3 * PLANE]);
 }
 
-constexpr int NBUF = 8;  // rho, u0, u1, u2, H, eta, p, T
+constexpr int NBUF = 8;  // rho, u0, u1, u2, H (TOTH: G), eta, p, T
 constexpr int NP2 = 18;  // 6 contravariant fluxes x 3 directions
 constexpr int NDTAB = 36;  // per CTA: D rows, then D^T rows, then D's row sums
 
@@ -111,7 +111,7 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
   const double kk = 0.5 * umag;
   const double e_int = Et * irho - 0.5 * umag;
   const double p = rho * (g - 1.0) * e_int;
-  const double Ht = a.prm.g_gm1 * p * irho + kk;  // h + k
+  const double Ht = TOTH ? Et + p : a.prm.g_gm1 * p * irho + kk;  // H = h + k (TOTH: G)
   const double T = p * irho * a.prm.inv_Rgas;
   // log(p / rho^gamma) as log p - gamma log rho (no pow)
   const double eta = (rho / (g - 1.0)) * (log(p) - g * log(rho));
@@ -162,7 +162,7 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
       Sm += wV * dr;
       Sn += wV * (n_ - eta);
       if constexpr (TOTH)
-        Se += wV * (r_ * H_ - rho * Ht);
+        Se += wV * (H_ - Ht);
       else
         Se += sr * (H_ - Ht);
 #pragma unroll
@@ -192,7 +192,7 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
   const double Rm = rho * divS + Sm;
   const double Rn = eta * divS + Sn;
   const double Rc = Rm + 0.25 * rho * sV;
-  const double Re = TOTH ? rho * Ht * divS + Se : Ht * Rc + Se;
+  const double Re = TOTH ? Ht * divS + Se : Ht * Rc + Se;
   double Rmo[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) Rmo[c] = uv[c] * Rc + Su[c];
@@ -251,8 +251,8 @@ __device__ __forceinline__ void rhs_fused_tile(const RhsArgs& a, int tile, unsig
   }
 }
 
-// Resident 64-thread element groups per SM the register budget must allow: 8 (128 registers; total
-// enthalpy spills 4 bytes).  Measured at 64^3 with whole values of u: 8 0.986 ms, 6 (154 registers) 1.087 ms;
+// Resident 64-thread element groups per SM the register budget must allow: 8 (128 registers, no
+// spill).  Measured at 64^3 with whole values of u: 8 0.986 ms, 6 (154 registers) 1.087 ms;
 // 10 (96 registers) would have spilled 244 bytes.
 #ifndef SOD_KR64_MIN_CTAS
 #define SOD_KR64_MIN_CTAS 8

@@ -112,3 +112,34 @@ def test_fused_mass_residual_of_a_shear(n):
     ref = assemble(m, conn, quartets(D, H, gpv, [c / R for c in Q], Q, R, 0 * R, 0 * R)[0])
     err = np.sqrt(np.mean((got - (ref / Ml).astype(float))**2))
     assert err < 2.0 * 2.0**-53 * rho / np.sqrt(2.0)
+
+
+def test_fused_total_enthalpy_energy_of_a_vortex():
+    """flag_total_enthalpy differentiates G = E + p.  Bound: u carries one rounding and G two, 0.3 * 2^-53 rms
+    each, which the rows of D (norm 3.9 rms) and the element size (n / pi) raise: 3.9 * 0.3 * sqrt(3) of u G n / pi.
+    Formed as rho (h + k), G adds the roundings of h, of k, of their sum and of the product."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from sod2d_refmap_b200 import build, mesh as M, solver as S
+    build.build()
+    n = 8
+    m, prm = M.periodic_box(n, jitter=0.05, seed=11), M.TGVParams(flag_total_enthalpy=1)
+    gm, s = S.Sod2dMesh(m, prm), S.Sod2dState.from_host(M.taylor_green_state(m, prm, 1e-2, seed=4), m.nelem)
+    s.mu_factor.fill_(0.0)
+    s.mu_e.fill_(0.0)
+    got = t2n(gm.rhs(s, precision=S.FP64)["Rener"])
+    conn, D, H, gpv, Ml = geometry(m, gm)
+    el = lambda t: t.cpu().numpy()[conn].reshape(-1, 4, 4, 4).astype(LD)
+    rho, q, E, g = el(s.rho), [el(s.q[c]) for c in range(3)], el(s.E), LD(prm.gamma_gas)
+    u = [c / rho for c in q]
+    G = E + (g - 1) * (E - rho * sum(c * c for c in u) / 2)
+
+    def grad(f):
+        d = [np.moveaxis(np.tensordot(D, f, axes=([1], [ax])), 0, ax) for ax in AXIS]
+        return [sum(H[c][k] * d[k] for k in range(3)) for c in range(3)]
+    div = lambda f: sum(grad(f[c])[c] for c in range(3))
+    ref = assemble(m, conn, gpv * (div([G * c for c in u]) + G * div(u) + sum(c * d for c, d in zip(u, grad(G)))) / 2) / Ml
+    err = np.sqrt(np.mean((got - ref).astype(float)**2))
+    uG = float(np.sqrt(np.mean(sum(c * c for c in u))) * np.mean(G))
+    assert err < 3.9 * 0.3 * np.sqrt(3.0) * 2.0**-53 * uG * n / np.pi
